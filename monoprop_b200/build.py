@@ -14,6 +14,7 @@ import os
 import subprocess
 import sys
 import sysconfig
+from concurrent.futures import ThreadPoolExecutor
 
 PKG = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(PKG)
@@ -35,15 +36,25 @@ def _sources(exts: tuple[str, ...]) -> list[str]:
 
 
 def build_engine(force: bool = False, verbose: bool = False) -> str:
-    cu = [os.path.join(CSRC, "mpx_engine.cu"), os.path.join(CSRC, "mpx_noalloc.cu"), os.path.join(CSRC, "mpx_batch.cu")]
+    cu = _sources((".cu",))
     deps = _sources((".cu", ".cuh", ".h")) + [os.path.join(ROOT, "include", "mpx.h")]
     if force or _stale(LIB, deps):
         cmd = [NVCC, *ARCH, "-O3", "-lineinfo", "-std=c++17", "--expt-relaxed-constexpr", "-Xcompiler", "-fPIC",
-               "-Xcompiler", "-fvisibility=hidden", "-shared", "-I", os.path.join(ROOT, "include"), *cu, "-o", LIB,
-               "-lcudart"]
+               "-Xcompiler", "-fvisibility=hidden", "-I", os.path.join(ROOT, "include")]
         if verbose:
             cmd.insert(1, "-Xptxas=-v")
-        subprocess.check_call(cmd)
+        objs = os.path.join(PKG, "build")
+        os.makedirs(objs, exist_ok=True)
+
+        def compile_one(src: str) -> str:
+            obj = os.path.join(objs, os.path.basename(src) + ".o")
+            if force or _stale(obj, [d for d in deps if not d.endswith(".cu") or d == src]):
+                subprocess.check_call([*cmd, "-c", src, "-o", obj])
+            return obj
+
+        with ThreadPoolExecutor(len(cu)) as pool:  # the translation units compile side by side
+            built = list(pool.map(compile_one, cu))
+        subprocess.check_call([NVCC, *ARCH, "-shared", *built, "-o", LIB, "-lcudart"])
     return LIB
 
 

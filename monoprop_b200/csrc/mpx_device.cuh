@@ -67,7 +67,10 @@ struct Counters {
     uint32_t stall;        // kNoStall, or the step index at which capacity ran out
     uint32_t err;          // nonzero: a bounded probe loop gave up (table inconsistent); results invalid
     unsigned long long rec_total; // pair records written by a recording forward pass (may exceed capacity)
+    uint32_t reason;       // why it stalled: kStallStore, or a window's kStallSector, kStallDense
+    uint32_t step;         // windows: the next step to run
 };
+constexpr uint32_t kStallStore = 0, kStallSector = 1, kStallDense = 2;
 
 // The key store is kept twice: as rows (keys, for the per-term work) and as bit-columns (cols, for the
 // anticommutation test). Column c (physical key bit c, c < 64W; c = 64W is the parity of |M|) is a
@@ -144,6 +147,22 @@ __device__ __forceinline__ void store_key(uint64_t *__restrict__ keys, uint64_t 
     }
 }
 
+// 32 x 32 bit transposition over a warp: lane r holds row r; afterwards bit r of lane c is bit c of row r.
+// Step j swaps the off-diagonal j x j blocks: the partner's row, rotated by j towards them, under a mask that
+// keeps the lane's own diagonal part (three instructions a step).
+__device__ __forceinline__ uint32_t transpose32(uint32_t x, int lane) {
+    uint32_t m = 0x0000FFFFu;
+#pragma unroll
+    for (int j = 16; j >= 1; j >>= 1) {
+        const bool up = (lane & j) != 0;
+        const uint32_t y = __shfl_xor_sync(0xFFFFFFFFu, x, j);
+        const uint32_t keep = up ? ~m : m;
+        x = (x & keep) | (__funnelshift_l(y, y, up ? 32 - j : j) & ~keep);
+        m ^= m << (j >> 1);
+    }
+    return x;
+}
+
 __device__ __forceinline__ int nc2(int n) { return (n * (n - 1)) >> 1; }
 
 // Anticommutation of M with the gate: Pauli parity(M & pair_swap(G)) (PauliAlgebra.h:80-83);
@@ -211,8 +230,8 @@ __device__ __forceinline__ bool keep_partner_mapped(const uint64_t (&p)[W], cons
 // Rotation phase of the sine branch M -> M^G.
 // Pauli: e = y(G) + y(M) - y(P) + 2 popcount(z(M) & x(G)); phase = -1 iff e mod 4 == 1 (PauliAlgebra.h:121-140).
 // Majorana: (-1)^parity(M & wmask) * {1,0,-1,0}[(C(|M|,2)+C(|G|,2)-C(|P|,2)+3) mod 4] (MajoranaAlgebra.h:104-122).
-template <int W, int BASIS>
-__device__ __forceinline__ int rotation_phase(const uint64_t (&m)[W], const uint64_t (&p)[W], const GateDesc &gd, int mpop,
+template <int W, int BASIS, class Gate>
+__device__ __forceinline__ int rotation_phase(const uint64_t (&m)[W], const uint64_t (&p)[W], const Gate &gd, int mpop,
                                               int ppop) {
     if constexpr (BASIS == 1) {
         int e = gd.gy;
@@ -256,5 +275,63 @@ __device__ __forceinline__ double state_score(const uint64_t (&m)[W], const Stat
 
 __device__ __forceinline__ uint8_t phase_code(int phase) { return phase > 0 ? 0 : (phase < 0 ? 1 : 2); }
 __device__ __forceinline__ double phase_value(uint8_t code) { return code == 0 ? 1.0 : (code == 1 ? -1.0 : 0.0); }
+
+// Writes the bit-columns of terms [lo, hi). A warp takes 8 consecutive column words (256 terms) at a
+// time: for each key word, two 32 x 32 bit transpositions per 32 terms build the 64 columns' words, which
+// then go out as whole 32-byte sectors (8 words of one column per 8 lanes) instead of 4-byte pieces of
+// 64W + 1 different columns. A word that starts below lo already holds valid bits for the terms below lo
+// (and zeros above) and is OR-ed; words outside [lo, hi) are not touched; every other word is assigned
+// whole (zeros above hi included). By all blocks of the grid, kBlock threads each.
+template <int W>
+__device__ __forceinline__ void columns_of(const Store &st, uint64_t lo, uint64_t hi, uint32_t (*s_col)[64][8]) {
+    if (hi <= lo) return;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint64_t w0 = lo >> 5, w1 = (hi + 31) >> 5;
+    const uint64_t g_first = w0 >> 3, g_end = (w1 + 7) >> 3;
+    const uint64_t n_warps = static_cast<uint64_t>(gridDim.x) * (kBlock / 32);
+    for (uint64_t grp = g_first + static_cast<uint64_t>(blockIdx.x) * (kBlock / 32) + warp; grp < g_end; grp += n_warps) {
+        const uint64_t j0 = grp * 8;
+        int pop[8];
+#pragma unroll
+        for (int g = 0; g < 8; ++g) pop[g] = 0;
+#pragma unroll 1
+        for (int w = 0; w < W; ++w) {
+#pragma unroll
+            for (int g = 0; g < 8; ++g) {
+                const uint64_t i = (j0 + g) * 32 + lane;
+                const uint64_t x = (i >= lo && i < hi) ? st.keys[i * W + w] : 0ULL;
+                pop[g] += __popcll(x);
+                const uint32_t lo_b = transpose32(static_cast<uint32_t>(x), lane);
+                const uint32_t hi_b = transpose32(static_cast<uint32_t>(x >> 32), lane);
+                s_col[warp][lane][g] = lo_b;
+                s_col[warp][lane + 32][g] = hi_b;
+            }
+            __syncwarp();
+            // 64 columns x 8 words: four columns per instruction, eight lanes per column
+#pragma unroll 4
+            for (int c4 = 0; c4 < 16; ++c4) {
+                const int c = c4 * 4 + (lane >> 3), g = lane & 7;
+                const uint64_t j = j0 + g;
+                if (j >= w0 && j < w1) {
+                    uint32_t *dst = st.cols + static_cast<uint64_t>(64 * w + c) * st.cstride + j;
+                    const uint32_t v = s_col[warp][c][g];
+                    *dst = (j * 32 < lo) ? (*dst | v) : v;
+                }
+            }
+            __syncwarp();
+        }
+        uint32_t par = 0;
+#pragma unroll
+        for (int g = 0; g < 8; ++g) {
+            const uint32_t b = __ballot_sync(0xFFFFFFFFu, pop[g] & 1);
+            if (lane == g) par = b;
+        }
+        const uint64_t j = j0 + lane;
+        if (lane < 8 && j >= w0 && j < w1) {
+            uint32_t *dst = st.cols + static_cast<uint64_t>(64 * W) * st.cstride + j;
+            *dst = (j * 32 < lo) ? (*dst | par) : par;
+        }
+    }
+}
 
 } // namespace mpx

@@ -23,6 +23,7 @@
 #include "../../include/mpx.h"
 #include "mpx_kernels.cuh"
 #include "mpx_small.cuh"
+#include "mpx_window.h"
 
 using namespace mpx;
 
@@ -151,6 +152,8 @@ struct mpx_engine {
         const uint32_t *w_anti;
         const uint32_t *r_src;
         uint64_t r_cap;
+        bool windows;
+        uint64_t launches; // kernels in it
         cudaGraphExec_t exec;
     };
     std::vector<GraphEntry> graphs;
@@ -178,6 +181,11 @@ struct mpx_engine {
     bool use_pdl = true; // programmatic dependent launch of the per-gate kernels
     bool use_graphs = true;
     bool small_path = true; // run small stores in one shared-memory block (mpx_small.cuh)
+    // gates in windows over the active terms (mpx_window.cuh); the scratch belongs to the store's capacity
+    WindowScratch ws{};
+    bool window_path = true;
+    bool window_nomem = false; // no room for the window scratch at this capacity: gate by gate
+    int sms = 0;
     std::string err;
 };
 
@@ -574,7 +582,7 @@ void launch_build(mpx_engine *e, uint64_t lo, uint64_t hi) {
     launch_table<W>(e, lo, hi);
     const uint64_t cblocks = std::min<uint64_t>((hi - lo + 32 * kBlock - 1) / (32 * kBlock) + 1,
                                                 static_cast<uint64_t>(e->grid));
-    k_columns<W><<<static_cast<unsigned>(cblocks), kBlock, 0, e->stream>>>(e->st, e->d_cnt, lo, hi, 0);
+    k_columns<W><<<static_cast<unsigned>(cblocks), kBlock, 0, e->stream>>>(e->st, lo, hi);
 }
 
 using GateFn = void (*)(mpx_engine *, const GateDesc *, uint32_t, uint32_t);
@@ -715,7 +723,83 @@ BuildFn pick_build(int W) {
 
 // Store buffers come from the engine's memory pool and go back to it stream-ordered (a plain cudaFree
 // would bypass the pool's bookkeeping, and the next engine would map fresh memory instead of reusing it).
+void free_window(mpx_engine *e) {
+    const WindowScratch &w = e->ws;
+    for (void *p : {static_cast<void *>(w.a_val), static_cast<void *>(w.a_mask), static_cast<void *>(w.a_idx),
+                    static_cast<void *>(w.a_bits), static_cast<void *>(w.a_lead), static_cast<void *>(w.fill),
+                    static_cast<void *>(w.slot_of), static_cast<void *>(w.act), static_cast<void *>(w.q_tgt),
+                    static_cast<void *>(w.ctl)})
+        dev_free(e, p);
+    e->ws = WindowScratch{};
+}
+
+uint32_t window_sectors(const mpx_engine *e) { return std::min<uint32_t>(kMaxSectors, static_cast<uint32_t>(e->sms * kSectorsPerSM)); }
+
+// List slots of the window path for capacity `cap`: above kLargeTerms terms at most a quarter is active when a
+// window starts (twice that leaves room for those that join), and each sector's last chunk may be partly used. (A window that needs more is run again
+// with a grown store.)
+uint64_t window_slots(const mpx_engine *e, uint64_t cap) {
+    const uint64_t terms = std::min(cap, std::max(cap / 2, kLargeTerms));
+    return (terms / kChunk + 2 * window_sectors(e) + 2) * kChunk;
+}
+
+// The window scratch of the store's capacity; false (and no scratch) when the device has no room for it.
+bool ensure_window(mpx_engine *e) {
+    if (e->ws.ctl != nullptr) return true;
+    if (e->window_nomem) return false;
+    WindowScratch w{};
+    w.slots = window_slots(e, e->st.cap);
+    const uint64_t terms = (e->st.cap + 255) / 256 * 256 + 256;
+    cudaError_t ce = cudaSuccess;
+    auto A = [&](auto **p, uint64_t count) {
+        if (ce == cudaSuccess) ce = dev_alloc(e, reinterpret_cast<void **>(p), count * sizeof(**p));
+        if (ce != cudaSuccess) *p = nullptr;
+    };
+    A(&w.a_val, w.slots);
+    A(&w.a_mask, w.slots);
+    A(&w.a_idx, w.slots);
+    A(&w.a_bits, w.slots / 32 * kWindow);
+    A(&w.a_lead, w.slots);
+    A(&w.fill, w.slots / kChunk);
+    A(&w.slot_of, terms);
+    A(&w.act, terms / 32);
+    A(&w.q_tgt, w.slots);
+    A(&w.ctl, 1);
+    e->ws = w;
+    if (ce == cudaSuccess) return true;
+    cudaGetLastError();
+    free_window(e);
+    e->window_nomem = true;
+    return false;
+}
+
+uint64_t window_bytes(const mpx_engine *e) {
+    if (e->ws.ctl == nullptr) return 0;
+    const uint64_t terms = (e->st.cap + 255) / 256 * 256 + 256;
+    return e->ws.slots * (2 * sizeof(uint64_t) + 2 * sizeof(uint32_t) + 1 + kWindow / 8) + terms * sizeof(uint32_t) + terms / 8;
+}
+
+WindowLaunch window_launch(mpx_engine *e, const CircuitDev &cd) {
+    WindowLaunch a{};
+    a.st = e->st;
+    a.sc = e->sc;
+    a.ws = e->ws;
+    a.cnt = e->d_cnt;
+    a.gates = cd.d_desc;
+    a.L = static_cast<uint32_t>(cd.n);
+    a.tr = e->tr;
+    a.stats = e->d_stats;
+    a.W = e->W;
+    a.basis = e->cfg.basis;
+    a.sectors = window_sectors(e);
+    a.threads = kSectorThreads;
+    a.blocks = static_cast<unsigned>(4 * e->sms);
+    a.stream = e->stream;
+    return a;
+}
+
 void free_store(mpx_engine *e) {
+    free_window(e);
     dev_free(e, e->st.keys);
     dev_free(e, e->st.coef);
     dev_free(e, e->st.table);
@@ -742,6 +826,8 @@ void clear_graphs(mpx_engine *e) {
 mpx_status alloc_store(mpx_engine *eng, uint64_t cap, uint64_t n_keep) {
     mpx_engine *e = eng;
     clear_graphs(e);
+    free_window(e);
+    e->window_nomem = false;
     ++e->store_gen;
     const int W = e->W;
     if (cap >= 0xFFFFFFF0ULL) return fail(eng, MPX_ERR_CAPACITY, "term capacity exceeds the 32-bit term index");
@@ -750,7 +836,8 @@ mpx_status alloc_store(mpx_engine *eng, uint64_t cap, uint64_t n_keep) {
     unsigned long long *table = nullptr;
     uint32_t *cols = nullptr;
     const uint64_t tcap = next_pow2(std::max<uint64_t>(cap << e->table_shift, 64));
-    const uint64_t q_cap = cap + (static_cast<uint64_t>(e->grid) * kWarps + 2) * 1024; // + region slack
+    const uint64_t q_cap = std::max<uint64_t>(cap + (static_cast<uint64_t>(e->grid) * kWarps + 2) * 1024, // + region slack
+                                              window_slots(e, cap));
     const uint64_t cstride = ((cap + 31) / 32 + 31) / 32 * 32; // 128-byte aligned columns
     Scratch nsc = e->sc;
     cudaError_t ce = cudaSuccess;
@@ -924,6 +1011,118 @@ mpx_status upload_circuit(mpx_engine *eng, const uint64_t *gen_words, const doub
     return MPX_OK;
 }
 
+// After a stall: room for n terms and the worst case of the stalled gates with headroom (four times the capacity,
+// fewer regrowths; at least double if that does not fit), and fresh counters.
+mpx_status grow_store(mpx_engine *eng, const Counters &snap) {
+    mpx_engine *e = eng;
+    const uint64_t n = snap.n, cap0 = e->st.cap;
+    mpx_status s = MPX_OK;
+    if (snap.reason == kStallDense) {
+        // nothing ran: the caller goes on gate by gate
+    }
+    else if (snap.reason == kStallSector) {
+        // a window's list was full: the store is as it was before the window, its table is not
+        MPX_CUDA(cudaMemsetAsync(e->st.table, 0xFF, (e->st.tmask + 1) * sizeof(unsigned long long), e->stream));
+        pick_table(e->W)(e, 0, n);
+    }
+    else {
+        s = alloc_store(e, std::max<uint64_t>(3 * n, 4 * cap0), n);
+        if (s == MPX_ERR_NOMEM) s = alloc_store(e, std::max<uint64_t>(3 * n, 2 * cap0), n);
+        if (s != MPX_OK) return s;
+    }
+    Counters fresh{};
+    fresh.n = n;
+    fresh.n0 = n;
+    fresh.stall = kNoStall;
+    fresh.err = snap.err;
+    fresh.rec_total = snap.rec_total; // a recording pass keeps its log offsets
+    MPX_CUDA(cudaMemcpyAsync(e->d_cnt, &fresh, sizeof(Counters), cudaMemcpyHostToDevice, e->stream));
+    MPX_CUDA(cudaStreamSynchronize(e->stream));
+    return MPX_OK;
+}
+
+// The next windows start at step `at`.
+cudaError_t start_windows(mpx_engine *e, uint64_t at) {
+    const uint32_t from = static_cast<uint32_t>(at);
+    const cudaError_t ce = cudaMemsetAsync(e->ws.ctl, 0, sizeof(WindowCtl), e->stream);
+    return ce != cudaSuccess ? ce : cudaMemcpyAsync(&e->d_cnt->step, &from, sizeof(from), cudaMemcpyHostToDevice, e->stream);
+}
+
+cudaError_t issue_window(mpx_engine *e, const WindowLaunch &w, uint64_t hi, cudaEvent_t *ev) {
+    if (ev) cudaEventRecord(ev[0], e->stream);
+    cudaError_t ce = window_close(w, static_cast<uint32_t>(hi));
+    if (ev) cudaEventRecord(ev[1], e->stream);
+    if (ce == cudaSuccess) ce = window_gates(w, static_cast<uint32_t>(hi));
+    if (ev) cudaEventRecord(ev[2], e->stream);
+    e->launches += 6;
+    return ce;
+}
+
+// Gates [*step, hi) in windows (mpx_window.cuh). A window's length is decided on the device, so the host issues
+// windows until one reports the end of the range, one ahead of the last report (unless the window in flight is
+// sure to end it). in_flight: a captured graph of windows has been launched and reports to h_snap[0]. *ran: how
+// many windows applied gates. Returns with *step < hi when windows cannot go on (no room for their scratch at
+// the grown capacity, or a sector's list over its limit): the caller goes on gate by gate.
+mpx_status run_windows(mpx_engine *eng, const CircuitDev &cd, uint64_t *step, uint64_t hi, bool in_flight, uint64_t *ran) {
+    mpx_engine *e = eng;
+    bool pending = in_flight, graph = in_flight;
+    uint64_t id = in_flight ? 1 : 0, slot = 0, known = *step;
+    size_t timed = 0;
+    if (!in_flight) MPX_CUDA(start_windows(e, known));
+    for (;;) {
+        bool issued = false;
+        const uint64_t least = !pending ? 0 : (graph ? hi : window_length(0, kWindow));
+        if (known + least < hi) {
+            MPX_CUDA(issue_window(e, window_launch(e, cd), hi, e->profile ? &e->pev[4 * timed] : nullptr));
+            timed += e->profile ? 1 : 0;
+            MPX_CUDA(cudaMemcpyAsync(&e->h_snap[id & 1], e->d_cnt, sizeof(Counters), cudaMemcpyDeviceToHost, e->stream));
+            MPX_CUDA(cudaEventRecord(e->ev[id & 1], e->stream));
+            issued = true;
+        }
+        if (pending) {
+            MPX_CUDA(cudaEventSynchronize(e->ev[slot]));
+            const Counters snap = e->h_snap[slot];
+            graph = false;
+            if (snap.stall != kNoStall) {
+                MPX_CUDA(cudaStreamSynchronize(e->stream));
+                ++e->launches;
+                MPX_CUDA(window_finish(window_launch(e, cd))); // the window before, if no later launch closed it yet
+                const mpx_status s = grow_store(e, snap);
+                if (s != MPX_OK) return s;
+                known = snap.stall;
+                if (snap.reason != kStallStore || !ensure_window(e)) {
+                    *step = known;
+                    return MPX_OK;
+                }
+                MPX_CUDA(start_windows(e, known));
+                pending = false;
+                ++id;
+                continue;
+            }
+            if (snap.step > known) ++*ran;
+            known = std::max<uint64_t>(known, snap.step);
+        }
+        if (!issued && known >= hi) break;
+        pending = issued;
+        slot = id & 1;
+        id += issued ? 1 : 0;
+    }
+    ++e->launches;
+    MPX_CUDA(window_finish(window_launch(e, cd))); // the last window's cos factors and counters
+    *step = hi;
+    if (e->profile) {
+        MPX_CUDA(cudaStreamSynchronize(e->stream));
+        for (size_t k = 0; k < timed; ++k) {
+            float a = 0.f, b = 0.f;
+            MPX_CUDA(cudaEventElapsedTime(&a, e->pev[4 * k], e->pev[4 * k + 1]));
+            MPX_CUDA(cudaEventElapsedTime(&b, e->pev[4 * k + 1], e->pev[4 * k + 2]));
+            e->t_sweep_ms += a;
+            e->t_resolve_ms += b;
+        }
+    }
+    return MPX_OK;
+}
+
 // Applies the uploaded gates last to first (Heisenberg; MonomialPropagator.inl:720-733). Gates are
 // issued in chunks; the counters after chunk k are inspected while chunk k+1 already runs, so the GPU
 // is never idle on a healthy run. A stalled step makes the rest of the queue no-ops; the host waits,
@@ -949,7 +1148,7 @@ mpx_status run_range(mpx_engine *eng, const CircuitDev &cd, uint64_t lo, uint64_
         }
     }
     const GateFn gate = pick_gate(e->W, e->cfg.basis);
-    constexpr uint64_t kChunk = 48;
+    constexpr uint64_t kChunkGates = 48;
     uint64_t step = lo;
     uint64_t chunk_id = 0;
     bool pending = false;
@@ -990,6 +1189,10 @@ mpx_status run_range(mpx_engine *eng, const CircuitDev &cd, uint64_t lo, uint64_
 
         }
     }
+    // Windows of gates over the active terms, or gate by gate: a tape, exact cos == 0 gates (their partner
+    // values need the kept pre-gate copy) and only_rotate_len_k take the per-gate kernels.
+    const bool windows = e->window_path && e->fwd_tape.w_anti == nullptr && !cd.any_cos_zero && !e->tr.has_len_k &&
+                         step < hi && ensure_window(e);
     const uint64_t gen0 = e->store_gen;
     // A gradient's forward pass is not captured: its tape buffers are allocated per call, so a captured
     // range would rarely match the next call's pointers and each miss would pay a new capture.
@@ -998,30 +1201,64 @@ mpx_status run_range(mpx_engine *eng, const CircuitDev &cd, uint64_t lo, uint64_
     const uint64_t glo = step;
     const bool graphable = e->use_graphs && !e->profile && cd.persistent && e->fwd_tape.w_anti == nullptr && glo < hi;
     bool replayed = false;
+    if (e->profile) e->t_sweep_ms = e->t_resolve_ms = e->t_columns_ms = 0.0;
     if (graphable) {
         for (const auto &g : e->graphs) {
-            if (g.circuit_id != cd.id || g.lo != glo || g.hi != hi || g.gen != gen0 || g.w_anti != e->fwd_tape.w_anti ||
-                g.r_src != e->fwd_tape.r_src || g.r_cap != e->fwd_tape.r_cap)
+            if (g.circuit_id != cd.id || g.lo != glo || g.hi != hi || g.gen != gen0 || g.windows != windows ||
+                g.w_anti != e->fwd_tape.w_anti || g.r_src != e->fwd_tape.r_src || g.r_cap != e->fwd_tape.r_cap)
                 continue;
             // One launch for the whole range; a gate that would overflow stalls the rest (no-ops), and the
-            // host resumes from it below exactly as after a chunk.
+            // host resumes from it below exactly as after a chunk. (New angles may need more windows than were
+            // captured; the host then goes on from where the graph ends.)
+            if (windows) MPX_CUDA(start_windows(e, step));
             MPX_CUDA(cudaGraphLaunch(g.exec, e->stream));
-            e->launches += 2 * (hi - glo);
+            e->launches += g.launches;
             ++e->graph_replays;
             MPX_CUDA(cudaMemcpyAsync(&e->h_snap[0], e->d_cnt, sizeof(Counters), cudaMemcpyDeviceToHost, e->stream));
             MPX_CUDA(cudaEventRecord(e->ev[0], e->stream));
-            step = hi;
-            pending = true;
-            pending_slot = 0;
-            chunk_id = 1;
+            if (!windows) {
+                step = hi;
+                pending = true;
+                pending_slot = 0;
+                chunk_id = 1;
+            }
             replayed = true;
             break;
         }
     }
+    // What ran, in order: `windows` windows that end at step `at`, then the steps up to `to` gate by gate.
+    struct Stretch {
+        uint64_t windows, at, to;
+    };
+    std::vector<Stretch> ran_as;
+    uint64_t stretch = hi; // end of the steps to run gate by gate before windows are tried again
+    uint64_t apart = kDenseGates; // doubled at every try that finds the store dense again
+    auto run_windows_from = [&](bool in_flight) -> mpx_status {
+        uint64_t ran = 0;
+        const mpx_status ws = run_windows(e, cd, &step, hi, in_flight, &ran);
+        apart = ran > 0 ? kDenseGates : 2 * apart;
+        stretch = e->profile ? hi : std::min(hi, step + apart); // one kind of timing after the other
+        ran_as.push_back({ran, step, stretch});
+        return ws;
+    };
+    if (windows) {
+        s = run_windows_from(replayed);
+        if (s != MPX_OK) return s;
+    }
+    const uint64_t by_gate = step; // the first step that runs gate by gate
     for (;;) {
         bool issued = false;
-        if (step < hi) {
-            const uint64_t stop = std::min(hi, step + kChunk);
+        if (step == stretch && stretch < hi && !pending) {
+            if (ensure_window(e)) {
+                s = run_windows_from(false);
+                if (s != MPX_OK) return s;
+            }
+            else {
+                stretch = hi;
+            }
+        }
+        if (step < stretch) {
+            const uint64_t stop = std::min(stretch, step + kChunkGates);
             for (uint64_t st = step; st < stop; ++st) {
                 gate(e, cd.d_desc, static_cast<uint32_t>(L - 1 - st), static_cast<uint32_t>(st));
             }
@@ -1038,32 +1275,18 @@ mpx_status run_range(mpx_engine *eng, const CircuitDev &cd, uint64_t lo, uint64_
             const Counters snap = e->h_snap[pending_slot];
             if (snap.stall != kNoStall) {
                 MPX_CUDA(cudaStreamSynchronize(e->stream));
-                const uint64_t at = snap.stall;
-                const uint64_t n = e->h_snap[pending_slot].n;
-                // room for the worst case of the stalled gate (2n) with headroom: four times the capacity
-                // (fewer regrowths), or, if that does not fit, at least double
-                const uint64_t cap0 = e->st.cap;
-                s = alloc_store(e, std::max<uint64_t>(3 * n, 4 * cap0), n);
-                if (s == MPX_ERR_NOMEM) s = alloc_store(e, std::max<uint64_t>(3 * n, 2 * cap0), n);
+                s = grow_store(e, snap);
                 if (s != MPX_OK) return s;
-                Counters fresh{};
-                fresh.n = n;
-                fresh.n0 = n;
-                fresh.stall = kNoStall;
-                fresh.err = snap.err;
-                fresh.rec_total = snap.rec_total; // a recording pass keeps its log offsets
-                MPX_CUDA(cudaMemcpyAsync(e->d_cnt, &fresh, sizeof(Counters), cudaMemcpyHostToDevice, e->stream));
-                MPX_CUDA(cudaStreamSynchronize(e->stream));
-                step = at;
+                step = snap.stall;
                 pending = false;
                 ++chunk_id;
                 continue;
             }
         }
-        if (!issued) break;
-        pending = true;
+        if (!issued && step >= hi) break;
+        pending = issued;
         pending_slot = chunk_id & 1;
-        ++chunk_id;
+        chunk_id += issued ? 1 : 0;
     }
     MPX_CUDA(cudaMemcpyAsync(e->h_cnt, e->d_cnt, sizeof(Counters), cudaMemcpyDeviceToHost, e->stream));
     MPX_CUDA(cudaStreamSynchronize(e->stream));
@@ -1072,11 +1295,31 @@ mpx_status run_range(mpx_engine *eng, const CircuitDev &cd, uint64_t lo, uint64_
         // the range ran without growing the store: capture it for the next call
         cudaGraph_t graph = nullptr;
         cudaGraphExec_t exec = nullptr;
+        const uint64_t launches0 = e->launches; // captured, not run
         bool ok = cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess;
         if (ok) {
-            for (uint64_t st = glo; st < hi; ++st) gate(e, cd.d_desc, static_cast<uint32_t>(L - 1 - st), static_cast<uint32_t>(st));
-            ok = cudaStreamEndCapture(e->stream, &graph) == cudaSuccess && graph != nullptr;
+            auto by_gates = [&](uint64_t from, uint64_t to) {
+                for (uint64_t st = from; st < to; ++st) gate(e, cd.d_desc, static_cast<uint32_t>(L - 1 - st), static_cast<uint32_t>(st));
+                e->launches += 2 * (to - from);
+            };
+            if (windows) {
+                const WindowLaunch w = window_launch(e, cd);
+                for (const Stretch &r : ran_as) {
+                    for (uint64_t k = 0; ok && k < r.windows; ++k) ok = issue_window(e, w, hi, nullptr) == cudaSuccess;
+                    if (r.to == r.at) continue;
+                    ok = ok && window_finish(w) == cudaSuccess &&
+                         window_handover(w, static_cast<uint32_t>(r.at), static_cast<uint32_t>(r.to)) == cudaSuccess;
+                    e->launches += 2;
+                    by_gates(r.at, r.to);
+                }
+            }
+            else {
+                by_gates(glo, hi);
+            }
+            ok = cudaStreamEndCapture(e->stream, &graph) == cudaSuccess && graph != nullptr && ok;
         }
+        const uint64_t captured = e->launches - launches0;
+        e->launches = launches0;
         ok = ok && cudaGraphInstantiate(&exec, graph, 0) == cudaSuccess;
         if (graph != nullptr) cudaGraphDestroy(graph);
         if (ok) {
@@ -1084,7 +1327,7 @@ mpx_status run_range(mpx_engine *eng, const CircuitDev &cd, uint64_t lo, uint64_
                 cudaGraphExecDestroy(e->graphs.front().exec);
                 e->graphs.erase(e->graphs.begin());
             }
-            e->graphs.push_back({cd.id, glo, hi, gen0, e->fwd_tape.w_anti, e->fwd_tape.r_src, e->fwd_tape.r_cap, exec});
+            e->graphs.push_back({cd.id, glo, hi, gen0, e->fwd_tape.w_anti, e->fwd_tape.r_src, e->fwd_tape.r_cap, windows, captured, exec});
         }
         else {
             e->use_graphs = false; // capture unavailable here: keep issuing kernels directly
@@ -1092,15 +1335,12 @@ mpx_status run_range(mpx_engine *eng, const CircuitDev &cd, uint64_t lo, uint64_
         cudaGetLastError();
     }
     if (e->profile) {
-        e->t_sweep_ms = e->t_resolve_ms = e->t_columns_ms = 0.0;
-        for (uint64_t st = lo; st < hi; ++st) {
-            float a = 0.f, b = 0.f, c = 0.f;
+        for (uint64_t st = by_gate; st < hi; ++st) {
+            float a = 0.f, b = 0.f;
             MPX_CUDA(cudaEventElapsedTime(&a, e->pev[4 * st], e->pev[4 * st + 1]));
             MPX_CUDA(cudaEventElapsedTime(&b, e->pev[4 * st + 1], e->pev[4 * st + 2]));
-            c = 0.0f; // no per-gate column launch: the resolve ORs the appended terms' bits
             e->t_sweep_ms += a;
             e->t_resolve_ms += b;
-            e->t_columns_ms += c;
         }
         e->n_sweep = hi - lo;
     }
@@ -2108,6 +2348,7 @@ mpx_status create_engine(const mpx_config *cfg, const uint64_t *obs_words, const
     // measured slower on the 100-qubit circuit: 8 blocks per SM 256 ms, 16 333 ms, against 214 ms.
     const int bps = cfg->blocks_per_sm > 0 ? std::min(cfg->blocks_per_sm, kSweepBlocksPerSM) : kSweepBlocksPerSM;
     e->grid = std::min(sms * bps, kMaxGrid);
+    e->sms = sms;
     e->table_shift = cfg->table_shift > 0 ? std::min(cfg->table_shift, 3) : 1;
     mpx_engine *eng = e;
     auto bail = [&](mpx_status st) {
@@ -2728,7 +2969,7 @@ mpx_status mpx_memory(mpx_engine *e, mpx_memory_info *out) {
     out->table_bytes = (e->st.tmask + 1) * sizeof(unsigned long long);
     out->column_bytes = (64 * W + 1) * e->st.cstride * sizeof(uint32_t);
     out->scratch_bytes = e->sc.q_cap * (sizeof(uint32_t) + sizeof(uint8_t) + sizeof(double)) +
-                         e->st.cstride * sizeof(uint32_t) + (e->aux_on ? e->st.cap * sizeof(double) : 0);
+                         e->st.cstride * sizeof(uint32_t) + (e->aux_on ? e->st.cap * sizeof(double) : 0) + window_bytes(e);
     out->initial_bytes = e->n_init * (W * sizeof(uint64_t) + sizeof(double)) +
                          e->n_start * (sizeof(uint32_t) + sizeof(double));
     const FrozenGraph &g = e->fg;
@@ -2773,6 +3014,7 @@ mpx_status clone_into(mpx_engine *e, mpx_engine *d) {
     d->pair_log = e->pair_log;
     d->rec_hint = e->rec_hint;
     d->small_path = e->small_path;
+    d->window_path = e->window_path;
     d->use_graphs = e->use_graphs;
     if (e->d_basis != nullptr) {
         const size_t bytes = static_cast<size_t>(64 * W) * W * sizeof(uint64_t);

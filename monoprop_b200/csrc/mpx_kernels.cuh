@@ -925,77 +925,11 @@ __global__ void __launch_bounds__(kBlock, kSweepBlocksPerSM) k_resolve(Store st,
     }
 }
 
-// Writes the bit-columns of terms [lo, hi). A warp takes 8 consecutive column words (256 terms) at a
-// time: for each key word, 64 ballots per 32 terms build the 64 columns' words in shared memory, which
-// then go out as whole 32-byte sectors (8 words of one column per 8 lanes) instead of 4-byte pieces of
-// 64W + 1 different columns. A word that starts below lo already holds valid bits for the terms below lo
-// (and zeros above) and is OR-ed; words outside [lo, hi) are not touched; every other word is assigned
-// whole (zeros above hi included). With from_counters the range is the current gate's appends [n0, n).
+// The bit-columns of terms [lo, hi) (columns_of).
 template <int W>
-__global__ void __launch_bounds__(kBlock) k_columns(Store st, const Counters *__restrict__ cnt, uint64_t lo,
-                                                     uint64_t hi, int from_counters) {
+__global__ void __launch_bounds__(kBlock) k_columns(Store st, uint64_t lo, uint64_t hi) {
     __shared__ uint32_t s_col[kWarps][64][8];
-    if (from_counters) {
-        if (cnt->stall != kNoStall) return;
-        lo = cnt->n0;
-        hi = cnt->n;
-    }
-    if (hi <= lo) return;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint64_t w0 = lo >> 5, w1 = (hi + 31) >> 5;
-    const uint64_t g_first = w0 >> 3, g_end = (w1 + 7) >> 3;
-    const uint64_t n_warps = static_cast<uint64_t>(gridDim.x) * kWarps;
-    for (uint64_t grp = g_first + static_cast<uint64_t>(blockIdx.x) * kWarps + warp; grp < g_end; grp += n_warps) {
-        const uint64_t j0 = grp * 8;
-        int pop[8];
-#pragma unroll
-        for (int g = 0; g < 8; ++g) pop[g] = 0;
-#pragma unroll 1
-        for (int w = 0; w < W; ++w) {
-#pragma unroll
-            for (int g = 0; g < 8; ++g) {
-                const uint64_t i = (j0 + g) * 32 + lane;
-                const uint64_t x = (i >= lo && i < hi) ? st.keys[i * W + w] : 0ULL;
-                pop[g] += __popcll(x);
-                uint32_t lo_b = 0, hi_b = 0;
-#pragma unroll
-                for (int b = 0; b < 32; ++b) {
-                    const uint32_t bl = __ballot_sync(0xFFFFFFFFu, (x >> b) & 1ULL);
-                    const uint32_t bh = __ballot_sync(0xFFFFFFFFu, (x >> (b + 32)) & 1ULL);
-                    if (lane == b) {
-                        lo_b = bl;
-                        hi_b = bh;
-                    }
-                }
-                s_col[warp][lane][g] = lo_b;
-                s_col[warp][lane + 32][g] = hi_b;
-            }
-            __syncwarp();
-            // 64 columns x 8 words: four columns per instruction, eight lanes per column
-#pragma unroll 4
-            for (int c4 = 0; c4 < 16; ++c4) {
-                const int c = c4 * 4 + (lane >> 3), g = lane & 7;
-                const uint64_t j = j0 + g;
-                if (j >= w0 && j < w1) {
-                    uint32_t *dst = st.cols + static_cast<uint64_t>(64 * w + c) * st.cstride + j;
-                    const uint32_t v = s_col[warp][c][g];
-                    *dst = (j * 32 < lo) ? (*dst | v) : v;
-                }
-            }
-            __syncwarp();
-        }
-        uint32_t par = 0;
-#pragma unroll
-        for (int g = 0; g < 8; ++g) {
-            const uint32_t b = __ballot_sync(0xFFFFFFFFu, pop[g] & 1);
-            if (lane == g) par = b;
-        }
-        const uint64_t j = j0 + lane;
-        if (lane < 8 && j >= w0 && j < w1) {
-            uint32_t *dst = st.cols + static_cast<uint64_t>(64 * W) * st.cstride + j;
-            *dst = (j * 32 < lo) ? (*dst | par) : par;
-        }
-    }
+    columns_of<W>(st, lo, hi, s_col);
 }
 
 // Inserts keys [lo, hi) into an empty-initialised table (construction, growth, reset).

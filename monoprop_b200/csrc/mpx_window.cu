@@ -1,0 +1,68 @@
+// mpx_window.cu -- launchers of the window kernels (mpx_window.cuh), one variant per key width, basis and
+// basis_change. A translation unit of its own: it compiles beside the engine's.
+#include "mpx_window.cuh"
+
+namespace mpx {
+namespace {
+
+template <int W, int B, bool MAPPED>
+cudaError_t sectors_launch(const WindowLaunch &a) {
+    const auto kernel = &k_window_gates<W, B, MAPPED>;
+    const size_t bytes = sizeof(GateShared<W>) + gate_lists_bytes(a.threads);
+    // the attribute belongs to the function and the device; setting it is cheap next to the window it runs
+    const cudaError_t ce = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
+    if (ce != cudaSuccess) return ce;
+    kernel<<<a.sectors, a.threads, bytes, a.stream>>>(a.st, a.sc, a.ws, a.cnt, a.gates, a.L, a.tr);
+    return cudaGetLastError();
+}
+
+template <int W>
+cudaError_t gates_w(const WindowLaunch &a, uint32_t hi) {
+    // the candidates' masks and sectors live where the queues and slot bits go later
+    auto *c_mask = reinterpret_cast<uint64_t *>(a.sc.q_val);
+    auto *c_sector = reinterpret_cast<uint16_t *>(a.ws.a_bits);
+    k_window_sample<W><<<kSampleBlocks, 256, 0, a.stream>>>(a.st, a.ws, a.sc.q_src, a.cnt, hi, a.sectors, a.tr);
+    k_window_count<W><<<a.blocks, 256, 0, a.stream>>>(a.st, a.ws, a.sc.q_src, c_mask, c_sector, a.cnt, hi, a.sectors, a.tr);
+    k_window_scatter<<<a.blocks, 256, 0, a.stream>>>(a.st, a.ws, a.sc.q_src, c_mask, c_sector, a.cnt, hi, a.sectors);
+    cudaError_t ce = cudaGetLastError();
+    if (ce != cudaSuccess) return ce;
+    if (a.basis == 1) ce = sectors_launch<W, 1, false>(a);
+    else if (a.tr.basis_rows != nullptr) ce = sectors_launch<W, 0, true>(a);
+    else ce = sectors_launch<W, 0, false>(a);
+    if (ce != cudaSuccess) return ce;
+    k_window_commit<W><<<a.blocks, kBlock, 0, a.stream>>>(a.st, a.ws, a.cnt);
+    return cudaGetLastError();
+}
+
+}  // namespace
+
+cudaError_t window_close(const WindowLaunch &a, uint32_t hi) {
+    k_window_close<<<a.blocks + 1, kCloseWarps * 32, 0, a.stream>>>(a.st, 64u * a.W, a.ws, a.sc.q_src, a.cnt, a.gates, a.L,
+                                                                hi, a.tr, a.stats);
+    return cudaGetLastError();
+}
+
+cudaError_t window_handover(const WindowLaunch &a, uint32_t at, uint32_t next) {
+    k_window_handover<<<1, 1, 0, a.stream>>>(a.cnt, at, next);
+    return cudaGetLastError();
+}
+
+cudaError_t window_finish(const WindowLaunch &a) {
+    const cudaError_t ce = window_close(a, 0);
+    return ce != cudaSuccess ? ce : cudaMemsetAsync(&a.ws.ctl->pending, 0, sizeof(uint32_t), a.stream);
+}
+
+cudaError_t window_gates(const WindowLaunch &a, uint32_t hi) {
+    switch (a.W) {
+    case 1: return gates_w<1>(a, hi);
+    case 2: return gates_w<2>(a, hi);
+    case 3: return gates_w<3>(a, hi);
+    case 4: return gates_w<4>(a, hi);
+    case 5: return gates_w<5>(a, hi);
+    case 6: return gates_w<6>(a, hi);
+    case 7: return gates_w<7>(a, hi);
+    default: return gates_w<8>(a, hi);
+    }
+}
+
+}  // namespace mpx
