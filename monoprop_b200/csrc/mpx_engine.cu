@@ -23,6 +23,7 @@
 #include "../../include/mpx.h"
 #include "mpx_kernels.cuh"
 #include "mpx_small.cuh"
+#include "mpx_replay.h"
 #include "mpx_window.h"
 
 using namespace mpx;
@@ -68,14 +69,9 @@ struct AdjointState {
     // only_rotate_len_k of the forward pass (0: none) and its outside-set bits over the final store
     uint32_t len_k = 0;
     uint32_t *longb = nullptr;
-    // a forward pass that logged everything the reverse sweep needs (log_ok: nothing overflowed): both
-    // pre-gate values of every recorded pair and the undo log; f_ubegin[st] = first undo record of step st
+    // a forward pass that logged everything the reverse sweep needs (log_ok: nothing overflowed): both pre-gate
+    // values of every recorded pair, and a checkpoint per replay window (ck_coef)
     double *r_vs = nullptr, *r_vt = nullptr;
-    uint32_t *f_uidx = nullptr;
-    double *f_uval = nullptr;
-    unsigned long long *f_utotal = nullptr;
-    uint64_t *f_ubegin = nullptr;
-    uint64_t f_ucap = 0;
     bool log_ok = false;
 };
 
@@ -101,6 +97,8 @@ struct FrozenGraph {
     // The recorded view of a propagation (the adjoint of that propagation) keeps the forward semantics:
     // such terms and partners are never scaled.
     bool forward_len_k = false;
+    ReplayPlan plan{}; // the pairs in replay order (mpx_replay.cuh), built at the first replay; windows = 0: none
+    bool no_plan = false; // no plan can be had (no room, or pairs the plan does not cover)
     Frozen view() const {
         return Frozen{src, tgt, code, p_begin, p_count, pared ? last : nullptr, forward_len_k ? longb : nullptr};
     }
@@ -159,6 +157,7 @@ struct mpx_engine {
     std::vector<GraphEntry> graphs;
     uint64_t store_gen = 0;
     uint64_t rec_hint = 0; // pair records the last recording forward pass needed (sizes the next log)
+    uint64_t ck_hint = 0; // terms of all replay windows' checkpoints in the last gradient forward pass
     uint64_t undo_hint = 0; // undo records (anticommuting terms over all gates) of the last gradient forward pass
     int64_t pair_log = -1; // mpx_set_pair_log: < 0 automatic, 0 off, > 0 fixed capacity
     uint64_t *d_basis = nullptr; // basis_change rows [2T][W] (tr.basis_rows points here when set)
@@ -1123,6 +1122,37 @@ mpx_status run_windows(mpx_engine *eng, const CircuitDev &cd, uint64_t *step, ui
     return MPX_OK;
 }
 
+// The pair log of a recording forward pass, four times as large (its first `used` records kept); left as it is
+// when it has a fixed size or the device has no room.
+void grow_pair_log(mpx_engine *e, uint64_t used) {
+    if (e->pair_log > 0) return;
+    const uint64_t cap = 4 * e->fwd_tape.r_cap;
+    uint32_t *src = nullptr, *tgt = nullptr;
+    int8_t *code = nullptr;
+    size_t free_b = device_available(e);
+    if (cap * 9 > free_b / 2) return;
+    cudaError_t ce = dev_alloc(e, reinterpret_cast<void **>(&src), cap * sizeof(uint32_t));
+    if (ce == cudaSuccess) ce = dev_alloc(e, reinterpret_cast<void **>(&tgt), cap * sizeof(uint32_t));
+    if (ce == cudaSuccess) ce = dev_alloc(e, reinterpret_cast<void **>(&code), cap * sizeof(int8_t));
+    if (ce == cudaSuccess) ce = cudaMemcpyAsync(src, e->adj.r_src, used * sizeof(uint32_t), cudaMemcpyDeviceToDevice, e->stream);
+    if (ce == cudaSuccess) ce = cudaMemcpyAsync(tgt, e->adj.r_tgt, used * sizeof(uint32_t), cudaMemcpyDeviceToDevice, e->stream);
+    if (ce == cudaSuccess) ce = cudaMemcpyAsync(code, e->adj.r_code, used, cudaMemcpyDeviceToDevice, e->stream);
+    if (ce != cudaSuccess) {
+        cudaGetLastError();
+        dev_free(e, src);
+        dev_free(e, tgt);
+        dev_free(e, code);
+        return;
+    }
+    dev_free(e, e->adj.r_src);
+    dev_free(e, e->adj.r_tgt);
+    dev_free(e, e->adj.r_code);
+    e->fwd_tape.r_src = e->adj.r_src = src;
+    e->fwd_tape.r_tgt = e->adj.r_tgt = tgt;
+    e->fwd_tape.r_code = e->adj.r_code = code;
+    e->fwd_tape.r_cap = cap;
+}
+
 // Applies the uploaded gates last to first (Heisenberg; MonomialPropagator.inl:720-733). Gates are
 // issued in chunks; the counters after chunk k are inspected while chunk k+1 already runs, so the GPU
 // is never idle on a healthy run. A stalled step makes the rest of the queue no-ops; the host waits,
@@ -1282,6 +1312,13 @@ mpx_status run_range(mpx_engine *eng, const CircuitDev &cd, uint64_t lo, uint64_
                 ++chunk_id;
                 continue;
             }
+            if (e->fwd_tape.r_src != nullptr && e->fwd_tape.r_vs == nullptr && step < hi &&
+                snap.rec_total > e->fwd_tape.r_cap / 4 && snap.rec_total <= e->fwd_tape.r_cap) {
+                // the pair log fills up: more room before the chunks after the one in flight (which may overflow it)
+                MPX_CUDA(cudaMemcpyAsync(e->h_cnt, e->d_cnt, sizeof(Counters), cudaMemcpyDeviceToHost, e->stream));
+                MPX_CUDA(cudaStreamSynchronize(e->stream));
+                if (e->h_cnt->rec_total <= e->fwd_tape.r_cap) grow_pair_log(e, e->h_cnt->rec_total);
+            }
         }
         if (!issued && step >= hi) break;
         pending = issued;
@@ -1396,12 +1433,17 @@ void free_adjoint(mpx_engine *e) {
     dev_free(e, e->adj.r_code);
     dev_free(e, e->adj.r_begin);
     dev_free(e, e->adj.longb);
-    for (void *p : {static_cast<void *>(e->adj.r_vs), static_cast<void *>(e->adj.r_vt),
-                    static_cast<void *>(e->adj.f_uidx), static_cast<void *>(e->adj.f_uval),
-                    static_cast<void *>(e->adj.f_utotal), static_cast<void *>(e->adj.f_ubegin)})
-        dev_free(e, p);
+    dev_free(e, e->adj.r_vs);
+    dev_free(e, e->adj.r_vt);
     e->adj = AdjointState{};
     e->fwd_tape = Tape{};
+}
+
+// Gates per replay window. Sectors stay balanced while the rank of the window's generators is well below the
+// number of key bits in use (2 per mode): on the 5x10 lattice 64 gates leave a few hundred cosets (busiest block
+// 8 times the mean), 25 leave it at 1.3 times; on the 6x6 Hubbard lattice 64 give 2.8, 36 give 1.6.
+uint32_t replay_window(const mpx_engine *e) {
+    return static_cast<uint32_t>(std::min<int>(kWindow, std::max(8, e->cfg.num_modes / 2)));
 }
 
 // Forward pass for the gradient: resets the store to the initial operator, propagates the circuit
@@ -1415,7 +1457,6 @@ mpx_status adjoint_forward(mpx_engine *eng, const CircuitDev &cd, uint64_t segme
     mpx_status s = load_initial(e);
     if (s != MPX_OK) return s;
     const uint64_t L = cd.n;
-    const uint64_t K = segment_gates == 0 ? std::max<uint64_t>(L, 1) : segment_gates;
     uint64_t n = e->n_init;
     const uint64_t n_warps = static_cast<uint64_t>(e->grid) * kWarps;
     MPX_CUDA(dev_alloc(e, reinterpret_cast<void **>(&e->adj.w_anti), std::max<uint64_t>(L, 1) * n_warps * sizeof(uint32_t)));
@@ -1423,7 +1464,7 @@ mpx_status adjoint_forward(mpx_engine *eng, const CircuitDev &cd, uint64_t segme
     // The pair log: sized by what the last recording pass needed (or the store capacity), checked after.
     if (e->pair_log != 0) {
         uint64_t r_cap = e->pair_log > 0 ? static_cast<uint64_t>(e->pair_log)
-                                         : std::max<uint64_t>({e->rec_hint + e->rec_hint / 4, e->st.cap, 1ULL << 16});
+                                         : std::max<uint64_t>({e->rec_hint + e->rec_hint / 4, e->st.cap, 1ULL << 20});
         // at most half of the free device memory, so that the store, the checkpoints and the backward
         // tape still fit (9 bytes per record)
         size_t free_b = 0, total_b = 0;
@@ -1444,45 +1485,29 @@ mpx_status adjoint_forward(mpx_engine *eng, const CircuitDev &cd, uint64_t segme
             cudaGetLastError(); // no room for a log: the backward pass replays with the streaming kernels
         }
     }
-    if (log_all && e->fwd_tape.r_src != nullptr && e->undo_hint > 0) {
+    // Logging everything the reverse sweep needs: both values of every pair, and a checkpoint per replay window
+    // (segments of that length). Needs the size of the pair log, which the previous pass of this engine gives.
+    uint64_t K = segment_gates == 0 ? std::max<uint64_t>(L, 1) : segment_gates;
+    if (log_all && e->window_path && e->fwd_tape.r_src != nullptr && e->undo_hint > 0 && !cd.any_cos_zero) {
         AdjointState &A = e->adj;
-        const uint64_t u_cap = e->undo_hint + e->undo_hint / 16 + (1ULL << 16);
         const uint64_t r_cap = e->fwd_tape.r_cap;
-        // large blocks come from power-of-two classes (dev_alloc)
-        const size_t need = next_pow2(u_cap * sizeof(uint32_t)) + next_pow2(u_cap * sizeof(double)) +
-                            2 * next_pow2(r_cap * sizeof(double)) + (L + 2) * sizeof(uint64_t);
+        // the values twice (as logged, and sorted for the reverse sweep), the sorted pairs, the checkpoints; large
+        // blocks come from power-of-two classes (dev_alloc)
+        const size_t need = 4 * next_pow2(r_cap * sizeof(double)) + 2 * next_pow2(r_cap * 17) + 2 * e->ck_hint * sizeof(double);
         // headroom for the store's growth and the backward pass's adjoint arrays
         const size_t reserve = (size_t{4} << 30) + static_cast<size_t>(e->st.cap) * 24;
         if (need + reserve <= device_available(e)) {
-            cudaError_t ce = dev_alloc(e, reinterpret_cast<void **>(&A.f_uidx), u_cap * sizeof(uint32_t));
-            if (ce == cudaSuccess) ce = dev_alloc(e, reinterpret_cast<void **>(&A.f_uval), u_cap * sizeof(double));
-            if (ce == cudaSuccess) ce = dev_alloc(e, reinterpret_cast<void **>(&A.r_vs), r_cap * sizeof(double));
+            cudaError_t ce = dev_alloc(e, reinterpret_cast<void **>(&A.r_vs), r_cap * sizeof(double));
             if (ce == cudaSuccess) ce = dev_alloc(e, reinterpret_cast<void **>(&A.r_vt), r_cap * sizeof(double));
-            if (ce == cudaSuccess) ce = dev_alloc(e, reinterpret_cast<void **>(&A.f_utotal), sizeof(unsigned long long));
-            if (ce == cudaSuccess) ce = dev_alloc(e, reinterpret_cast<void **>(&A.f_ubegin), (L + 1) * sizeof(uint64_t));
-            if (ce == cudaSuccess) ce = cudaMemsetAsync(A.f_utotal, 0, sizeof(unsigned long long), e->stream);
-            if (ce == cudaSuccess) ce = cudaMemsetAsync(A.f_ubegin, 0, (L + 1) * sizeof(uint64_t), e->stream);
             if (ce == cudaSuccess) {
-                A.f_ucap = u_cap;
                 e->fwd_tape.r_vs = A.r_vs;
                 e->fwd_tape.r_vt = A.r_vt;
-                e->fwd_tape.f_uidx = A.f_uidx;
-                e->fwd_tape.f_uval = A.f_uval;
-                e->fwd_tape.f_utotal = A.f_utotal;
-                e->fwd_tape.f_ubegin = A.f_ubegin;
-                e->fwd_tape.f_ucap = u_cap;
+                K = replay_window(e);
             }
             else {
                 cudaGetLastError(); // no room after all: the backward pass replays segments
-                for (void *p : {static_cast<void *>(A.r_vs), static_cast<void *>(A.r_vt),
-                                static_cast<void *>(A.f_uidx), static_cast<void *>(A.f_uval),
-                                static_cast<void *>(A.f_utotal), static_cast<void *>(A.f_ubegin)})
-                    dev_free(e, p);
+                dev_free(e, A.r_vs);
                 A.r_vs = A.r_vt = nullptr;
-                A.f_uidx = nullptr;
-                A.f_uval = nullptr;
-                A.f_utotal = nullptr;
-                A.f_ubegin = nullptr;
             }
         }
     }
@@ -1505,12 +1530,7 @@ mpx_status adjoint_forward(mpx_engine *eng, const CircuitDev &cd, uint64_t segme
         e->adj.rec_ok = e->adj.r_total <= e->fwd_tape.r_cap;
         e->rec_hint = std::max(e->rec_hint, e->adj.r_total);
     }
-    if (e->fwd_tape.f_utotal != nullptr) {
-        unsigned long long u_total = 0;
-        MPX_CUDA(cudaMemcpyAsync(&u_total, e->fwd_tape.f_utotal, sizeof(u_total), cudaMemcpyDeviceToHost, e->stream));
-        MPX_CUDA(cudaStreamSynchronize(e->stream));
-        e->adj.log_ok = e->adj.rec_ok && u_total <= e->adj.f_ucap;
-    }
+    e->adj.log_ok = e->adj.rec_ok && e->adj.r_vs != nullptr;
     e->fwd_tape = Tape{};
     if (e->tr.has_len_k) {
         // only_rotate_len_k: which terms of the final store lie outside every gate's rotation set
@@ -1539,98 +1559,9 @@ mpx_status adjoint_forward(mpx_engine *eng, const CircuitDev &cd, uint64_t segme
     uint64_t undo = 0;
     for (uint64_t st = 0; st < L; ++st) undo += e->adj.stats[4 * st + 1];
     if (log_all) e->undo_hint = undo;
-    return MPX_OK;
-}
-
-// Reverse sweep over the logs of a forward pass that logged everything (AdjointState::log_ok): no
-// checkpoint, no replay. Pair members keep their undo records (the sweep wrote them before the resolve
-// knew the pairs), so each gate runs the pairs kernel, which marks them done, then the undo kernel.
-mpx_status adjoint_backward_logged(mpx_engine *eng, const CircuitDev &cd, double *grad_angles) {
-    mpx_engine *e = eng;
-    AdjointState &A = e->adj;
-    const uint64_t L = A.L, nf = A.n_final;
-    std::vector<uint64_t> ub(L + 1), rb(L);
-    MPX_CUDA(cudaMemcpyAsync(ub.data(), A.f_ubegin, (L + 1) * sizeof(uint64_t), cudaMemcpyDeviceToHost, e->stream));
-    MPX_CUDA(cudaMemcpyAsync(rb.data(), A.r_begin, L * sizeof(uint64_t), cudaMemcpyDeviceToHost, e->stream));
-    MPX_CUDA(cudaStreamSynchronize(e->stream));
-    std::vector<unsigned long long> cnts(2 * L);
-    for (uint64_t st = 0; st < L; ++st) {
-        cnts[st] = ub[st + 1] - ub[st];
-        cnts[L + st] = (st + 1 < L ? rb[st + 1] : A.r_total) - rb[st];
-    }
-    unsigned long long *d_cnts = nullptr; // u_cnt | p_cnt
-    double *lam = nullptr, *grad = nullptr, *gpart = nullptr;
-    uint32_t *done = nullptr;
-    cudaError_t ce = cudaSuccess;
-    auto A_ = [&](void **ptr, size_t bytes) {
-        if (ce == cudaSuccess) ce = dev_alloc(e, ptr, std::max<size_t>(bytes, 16));
-    };
-    A_(reinterpret_cast<void **>(&d_cnts), 2 * L * sizeof(unsigned long long));
-    A_(reinterpret_cast<void **>(&lam), nf * sizeof(double));
-    A_(reinterpret_cast<void **>(&grad), L * sizeof(double));
-    A_(reinterpret_cast<void **>(&done), ((nf + 31) / 32) * sizeof(uint32_t));
-    A_(reinterpret_cast<void **>(&gpart), (2 * static_cast<size_t>(e->grid) + 1) * sizeof(double));
-    auto release = [&]() {
-        for (void *ptr : {static_cast<void *>(d_cnts), static_cast<void *>(lam), static_cast<void *>(grad),
-                          static_cast<void *>(done), static_cast<void *>(gpart)})
-            dev_free(e, ptr);
-    };
-    if (ce != cudaSuccess) {
-        cudaGetLastError();
-        release();
-        return fail(eng, MPX_ERR_NOMEM, std::string("gradient allocation failed: ") + cudaGetErrorString(ce));
-    }
-#define MPX_CUDA_REL(call)                                                                                          \
-    do {                                                                                                            \
-        cudaError_t e2_ = (call);                                                                                   \
-        if (e2_ != cudaSuccess) {                                                                                   \
-            release();                                                                                              \
-            return fail(eng, MPX_ERR_CUDA, std::string(#call ": ") + cudaGetErrorString(e2_));                     \
-        }                                                                                                           \
-    } while (0)
-    MPX_CUDA_REL(cudaMemcpyAsync(d_cnts, cnts.data(), 2 * L * sizeof(unsigned long long), cudaMemcpyHostToDevice,
-                                 e->stream));
-    MPX_CUDA_REL(cudaMemsetAsync(grad, 0, L * sizeof(double), e->stream));
-    MPX_CUDA_REL(cudaMemsetAsync(done, 0, std::max<uint64_t>((nf + 31) / 32, 1) * sizeof(uint32_t), e->stream));
-    const GradPartials gp{gpart, reinterpret_cast<unsigned int *>(gpart + 2 * static_cast<size_t>(e->grid))};
-    MPX_CUDA_REL(cudaMemsetAsync(gp.arrivals, 0, sizeof(unsigned int), e->stream));
-    if (e->schr) {
-        MPX_CUDA_REL(cudaMemsetAsync(lam, 0, std::max<uint64_t>(nf, 1) * sizeof(double), e->stream));
-        if (e->n_obs > 0 && nf > 0) {
-            pick_lookup(e->W)(e, e->d_obs_keys, e->n_obs, nf, e->d_obs_idx);
-            k_scatter<<<static_cast<unsigned>(std::min<uint64_t>((e->n_obs + 255) / 256, 4096)), 256, 0, e->stream>>>(
-                lam, e->d_obs_idx, e->d_obs_coef, e->n_obs);
-        }
-    }
-    else {
-        pick_adj_init(e->W, e->cfg.basis)(e, lam, 0, nf);
-    }
-    Tape tp{};
-    tp.u_idx = A.f_uidx;
-    tp.u_val = A.f_uval;
-    tp.u_base = A.f_ubegin;
-    tp.u_cnt = d_cnts;
-    tp.p_src = A.r_src;
-    tp.p_tgt = A.r_tgt;
-    tp.p_code = A.r_code;
-    tp.p_vs = A.r_vs;
-    tp.p_vt = A.r_vt;
-    tp.p_base = A.r_begin;
-    tp.p_cnt = d_cnts + L;
-    for (uint64_t st = L; st-- > 0;) {
-        const uint32_t gate = static_cast<uint32_t>(L - 1 - st);
-        launch_dep(e, &k_adj_pairs, tp, static_cast<const GateDesc *>(cd.d_desc), gate, static_cast<uint32_t>(st), lam,
-                   done, gp);
-        launch_dep(e, &k_adj_undo, tp, static_cast<const GateDesc *>(cd.d_desc), gate, static_cast<uint32_t>(st), lam,
-                   done, gp, grad);
-    }
-    e->launches += 2 * L + 1;
-    MPX_CUDA_REL(cudaGetLastError());
-    MPX_CUDA_REL(cudaMemcpyAsync(grad_angles, grad, L * sizeof(double), cudaMemcpyDeviceToHost, e->stream));
-    MPX_CUDA_REL(cudaStreamSynchronize(e->stream));
-#undef MPX_CUDA_REL
-    release();
-    MPX_CUDA(cudaStreamSynchronize(e->stream));
+    e->ck_hint = 0;
+    const uint64_t window = replay_window(e);
+    for (uint64_t st = 0; st < L; st += window) e->ck_hint += e->adj.stats[4 * st];
     return MPX_OK;
 }
 
@@ -1655,6 +1586,232 @@ mpx_status replay_start_tail(mpx_engine *eng, uint64_t lo, uint64_t hi, bool wit
     return MPX_OK;
 }
 
+// ----- windowed replay (mpx_replay.cuh) -----------------------------------------------------------------
+
+void free_plan(mpx_engine *e, ReplayPlan &p) {
+    for (void *q : {static_cast<void *>(p.src), static_cast<void *>(p.tgt), static_cast<void *>(p.code),
+                    static_cast<void *>(p.mask), static_cast<void *>(p.seg), static_cast<void *>(p.comm)})
+        dev_free(e, q);
+    p = ReplayPlan{};
+}
+
+ReplayLaunch replay_launch(const mpx_engine *e, const CircuitDev &cd, const FrozenGraph &g) {
+    return ReplayLaunch{e->st, g.forward_len_k ? g.longb : nullptr, cd.d_desc, static_cast<uint32_t>(cd.n), e->W, static_cast<unsigned>(4 * e->sms), e->stream};
+}
+
+// Sorts the structure's pairs into replay order. in_vs / in_vt with vs / vt: the pairs' logged values, sorted
+// along. Leaves p empty (MPX_OK) when the device has no room or the pairs have no 32-bit numbers.
+mpx_status build_plan(mpx_engine *eng, const CircuitDev &cd, const FrozenGraph &g, const double *in_vs, const double *in_vt,
+                      double *vs, double *vt, ReplayPlan &p) {
+    mpx_engine *e = eng;
+    p = ReplayPlan{};
+    const uint64_t L = g.L;
+    if (L == 0 || g.src == nullptr) return MPX_OK;
+    std::vector<uint64_t> begin(L);
+    MPX_CUDA(cudaMemcpyAsync(begin.data(), g.p_begin, L * sizeof(uint64_t), cudaMemcpyDeviceToHost, e->stream));
+    MPX_CUDA(cudaStreamSynchronize(e->stream));
+    // pairs of every window, and its range of the log (with the places a replayed build's log leaves empty)
+    uint64_t total = 0;
+    const uint32_t K = replay_window(e), n_win = static_cast<uint32_t>((L + K - 1) / K);
+    std::vector<uint64_t> range(n_win, 0);
+    std::vector<uint32_t> base(n_win, 0);
+    for (uint64_t st = 0; st < L; ++st) {
+        if (st % K == 0) base[st / K] = static_cast<uint32_t>(total);
+        total += g.count[st];
+        range[st / K] = begin[st] + g.count[st] - begin[st / K * K];
+        if (total >= 0xFFFFFFFFull) return MPX_OK;
+    }
+    const uint64_t places = begin[L - 1] + g.count[L - 1];
+    ReplayPlan q{};
+    ReplaySort so{};
+    q.gates = K;
+    q.windows = n_win;
+    q.sectors = window_sectors(e);
+    const uint64_t slots = static_cast<uint64_t>(q.sectors) * K;
+    cudaError_t ce = cudaSuccess;
+    auto A = [&](auto **ptr, uint64_t n) {
+        if (ce == cudaSuccess) ce = dev_alloc(e, reinterpret_cast<void **>(ptr), std::max<uint64_t>(n, 4) * sizeof(**ptr));
+        if (ce != cudaSuccess) *ptr = nullptr;
+    };
+    A(&q.src, total);
+    A(&q.tgt, total);
+    A(&q.code, total);
+    A(&q.mask, total);
+    A(&q.seg, n_win * (slots + 1));
+    A(&q.comm, static_cast<uint64_t>(n_win) * kWindow);
+    A(&so.tables, n_win);
+    A(&so.cursor, n_win * slots);
+    A(&so.base, n_win);
+    A(&so.c_mask, places);
+    A(&so.c_sector, places);
+    if (ce == cudaSuccess)
+        ce = cudaMemcpyAsync(so.base, base.data(), n_win * sizeof(uint32_t), cudaMemcpyHostToDevice, e->stream);
+    const ReplayLaunch a = replay_launch(e, cd, g);
+    if (ce == cudaSuccess) ce = cudaMemsetAsync(q.seg, 0, n_win * (slots + 1) * sizeof(uint32_t), e->stream);
+    if (ce == cudaSuccess) ce = replay_tables(a, q, so);
+    for (uint32_t w = 0; ce == cudaSuccess && w < n_win; ++w) 
+        ce = replay_count(a, q, so, w, g.src, g.p_begin, g.p_count, begin[w * K], range[w]);
+    if (ce == cudaSuccess) ce = replay_prefix(a, q, so);
+    for (uint32_t w = 0; ce == cudaSuccess && w < n_win; ++w)
+        ce = replay_scatter(a, q, so, w, g.src, g.tgt, g.code, in_vs, in_vt, vs, vt, g.p_begin, g.p_count, begin[w * K],
+                            range[w]);
+    e->launches += 2 + 2 * n_win;
+    for (void *ptr : {static_cast<void *>(so.tables), static_cast<void *>(so.cursor), static_cast<void *>(so.base),
+                      static_cast<void *>(so.c_mask),
+                      static_cast<void *>(so.c_sector)})
+        dev_free(e, ptr);
+    if (ce != cudaSuccess) {
+        free_plan(e, q);
+        if (ce != cudaErrorMemoryAllocation) MPX_CUDA(ce);
+        cudaGetLastError();
+        return MPX_OK;
+    }
+    p = q;
+    return MPX_OK;
+}
+
+// The plan of the engine's graph, built at its first replay; nullptr when the graph replays gate by gate (see
+// build_plan) and when a gate has cos == 0 (kappa needs the quotient).
+const ReplayPlan *graph_plan(mpx_engine *e, const CircuitDev &cd, FrozenGraph &g) {
+    if (!e->window_path || cd.any_cos_zero || g.no_plan) return nullptr;
+    if (g.plan.windows == 0) {
+        if (build_plan(e, cd, g, nullptr, nullptr, nullptr, nullptr, g.plan) != MPX_OK || g.plan.windows == 0) {
+            g.no_plan = true;
+            return nullptr;
+        }
+    }
+    return &g.plan;
+}
+
+// lambda of the final state: the observable's weights (Schrodinger), or the reference-state scores.
+mpx_status final_adjoint(mpx_engine *eng, double *lam, uint64_t nf) {
+    mpx_engine *e = eng;
+    if (e->schr) {
+        MPX_CUDA(cudaMemsetAsync(lam, 0, std::max<uint64_t>(nf, 1) * sizeof(double), e->stream));
+        if (e->n_obs > 0 && nf > 0) {
+            pick_lookup(e->W)(e, e->d_obs_keys, e->n_obs, nf, e->d_obs_idx);
+            k_scatter<<<static_cast<unsigned>(std::min<uint64_t>((e->n_obs + 255) / 256, 4096)), 256, 0, e->stream>>>(
+                lam, e->d_obs_idx, e->d_obs_coef, e->n_obs);
+        }
+    }
+    else {
+        pick_adj_init(e->W, e->cfg.basis)(e, lam, 0, nf);
+    }
+    MPX_CUDA(cudaGetLastError());
+    return MPX_OK;
+}
+
+// The gradient of the frozen structure g at the circuit's angles from the state in the store (every term of the
+// final store at its starting value): the plan replayed forward with the pairs' values and a coefficient
+// checkpoint per window logged, then the reverse sweep. Leaves the replayed state in the store. *done = false
+// (MPX_OK, store untouched) when the device has no room for the logs.
+mpx_status replay_gradient(mpx_engine *eng, const CircuitDev &cd, const FrozenGraph &g, const ReplayPlan &p,
+                           double *grad_angles, bool *done) {
+    mpx_engine *e = eng;
+    *done = false;
+    const uint64_t L = g.L, nf = g.n_final;
+    uint64_t pairs = 0;
+    for (const uint64_t c : g.count) pairs += c;
+    double *vs = nullptr, *vt = nullptr, *lam = nullptr, *grad = nullptr;
+    uint8_t *mark = nullptr; // forward: gates applied per term; backward: its earliest pair
+    std::vector<double *> ck(p.windows, nullptr);
+    cudaError_t ce = cudaSuccess;
+    auto A = [&](auto **ptr, uint64_t n) {
+        if (ce == cudaSuccess) ce = dev_alloc(e, reinterpret_cast<void **>(ptr), std::max<uint64_t>(n, 4) * sizeof(**ptr));
+        if (ce != cudaSuccess) *ptr = nullptr;
+    };
+    A(&vs, pairs);
+    A(&vt, pairs);
+    A(&lam, nf);
+    A(&grad, L);
+    A(&mark, nf);
+    for (uint32_t w = 0; w < p.windows; ++w) A(&ck[w], g.n0[static_cast<uint64_t>(w) * p.gates]);
+    auto release = [&]() {
+        for (void *q : {static_cast<void *>(vs), static_cast<void *>(vt), static_cast<void *>(lam), static_cast<void *>(grad),
+                        static_cast<void *>(mark)})
+            dev_free(e, q);
+        for (double *q : ck) dev_free(e, q);
+    };
+    if (ce != cudaSuccess) {
+        cudaGetLastError();
+        release();
+        return MPX_OK;
+    }
+    const ReplayLaunch a = replay_launch(e, cd, g);
+    const uint64_t n_first = g.n0[0];
+    ce = cudaMemsetAsync(mark, 0, std::max<uint64_t>(nf, 4), e->stream);
+    if (ce == cudaSuccess) ce = cudaMemsetAsync(grad, 0, L * sizeof(double), e->stream);
+    if (ce == cudaSuccess && n_first > 0)
+        ce = cudaMemcpyAsync(ck[0], e->st.coef, n_first * sizeof(double), cudaMemcpyDeviceToDevice, e->stream);
+    auto end_of = [&](uint32_t w) { return w + 1 < p.windows ? g.n0[static_cast<uint64_t>(w + 1) * p.gates] : nf; };
+    for (uint32_t w = 0; ce == cudaSuccess && w < p.windows; ++w)
+        ce = replay_forward(a, p, w, end_of(w), mark, vs, vt, w + 1 < p.windows ? ck[w + 1] : nullptr);
+    mpx_status s = ce == cudaSuccess ? final_adjoint(e, lam, nf) : MPX_OK;
+    for (uint32_t w = p.windows; ce == cudaSuccess && s == MPX_OK && w-- > 0;)
+        ce = replay_reverse(a, p, w, g.n0[static_cast<uint64_t>(w) * p.gates], lam, mark, vs, vt, ck[w], grad);
+    e->launches += 4 * p.windows + 1;
+    if (ce == cudaSuccess && s == MPX_OK)
+        ce = cudaMemcpyAsync(grad_angles, grad, L * sizeof(double), cudaMemcpyDeviceToHost, e->stream);
+    if (ce == cudaSuccess) ce = cudaStreamSynchronize(e->stream);
+    release();
+    if (s != MPX_OK) return s;
+    MPX_CUDA(ce);
+    *done = true;
+    return MPX_OK;
+}
+
+// Reverse sweep over the logs of a forward pass that logged everything (AdjointState::log_ok): the pairs are
+// sorted into replay order with their values, and the windows swept from the checkpoints at their starts. No
+// replay. *done = false (MPX_OK): no room for the sorted pairs, the caller replays the segments.
+mpx_status adjoint_backward_logged(mpx_engine *eng, const CircuitDev &cd, const FrozenGraph &g, double *grad_angles,
+                                   bool *done) {
+    mpx_engine *e = eng;
+    AdjointState &A = e->adj;
+    *done = false;
+    const uint64_t L = A.L, nf = A.n_final;
+    double *vs = nullptr, *vt = nullptr, *lam = nullptr, *grad = nullptr;
+    uint8_t *mark = nullptr;
+    ReplayPlan p{};
+    cudaError_t ce = cudaSuccess;
+    auto alloc = [&](auto **ptr, uint64_t n) {
+        if (ce == cudaSuccess) ce = dev_alloc(e, reinterpret_cast<void **>(ptr), std::max<uint64_t>(n, 4) * sizeof(**ptr));
+        if (ce != cudaSuccess) *ptr = nullptr;
+    };
+    alloc(&vs, A.r_total);
+    alloc(&vt, A.r_total);
+    alloc(&lam, nf);
+    alloc(&grad, L);
+    alloc(&mark, nf);
+    auto release = [&]() {
+        for (void *q : {static_cast<void *>(vs), static_cast<void *>(vt), static_cast<void *>(lam), static_cast<void *>(grad),
+                        static_cast<void *>(mark)})
+            dev_free(e, q);
+        free_plan(e, p);
+    };
+    mpx_status s = MPX_OK;
+    if (ce == cudaSuccess) s = build_plan(e, cd, g, A.r_vs, A.r_vt, vs, vt, p);
+    if (ce != cudaSuccess || s != MPX_OK || p.windows == 0 || p.windows != A.ck_coef.size()) {
+        cudaGetLastError();
+        release();
+        return s;
+    }
+    ce = cudaMemsetAsync(mark, 0, std::max<uint64_t>(nf, 4), e->stream);
+    if (ce == cudaSuccess) ce = cudaMemsetAsync(grad, 0, L * sizeof(double), e->stream);
+    if (ce == cudaSuccess) s = final_adjoint(e, lam, nf);
+    const ReplayLaunch a = replay_launch(e, cd, g);
+    for (uint32_t w = p.windows; ce == cudaSuccess && s == MPX_OK && w-- > 0;)
+        ce = replay_reverse(a, p, w, A.ck_n[w], lam, mark, vs, vt, A.ck_coef[w], grad);
+    e->launches += 2 * p.windows + 1;
+    if (ce == cudaSuccess && s == MPX_OK)
+        ce = cudaMemcpyAsync(grad_angles, grad, L * sizeof(double), cudaMemcpyDeviceToHost, e->stream);
+    if (ce == cudaSuccess) ce = cudaStreamSynchronize(e->stream);
+    release();
+    if (s != MPX_OK) return s;
+    MPX_CUDA(ce);
+    *done = true;
+    return MPX_OK;
+}
+
 // Reverse sweep: per segment (last first) restore its checkpoint, replay it logging the tape, then walk
 // its gates backwards. grad_angles[l] = dE/d(angle_l) for circuit layer l (angle = theta[map] * g).
 // With fg == nullptr: the gradient of the last mpx_adjoint_forward (segments replayed with the
@@ -1666,6 +1823,41 @@ mpx_status adjoint_backward(mpx_engine *eng, const CircuitDev &cd, double *grad_
     const uint64_t L = A.L;
     const uint64_t nf = A.n_final;
     const size_t S = A.seg_lo.size();
+    if (fg != nullptr && S == 1) {
+        // one segment: the windowed replay, when the structure has a plan and its logs fit
+        ReplayPlan own{};
+        const ReplayPlan *plan = nullptr;
+        if (fg == &e->fg) {
+            plan = graph_plan(e, cd, e->fg);
+        }
+        else if (e->window_path && !cd.any_cos_zero) {
+            const mpx_status ps = build_plan(e, cd, *fg, nullptr, nullptr, nullptr, nullptr, own);
+            if (ps != MPX_OK) return ps;
+            plan = own.windows != 0 ? &own : nullptr;
+        }
+        bool done = false;
+        if (plan != nullptr) {
+            const uint64_t n = A.ck_n[0];
+            mpx_status rs = MPX_OK;
+            if (n > 0)
+                MPX_CUDA(cudaMemcpyAsync(e->st.coef, A.ck_coef[0], n * sizeof(double), cudaMemcpyDeviceToDevice, e->stream));
+            if (nf > n) rs = replay_start_tail(e, n, nf, fg == &e->fg);
+            if (rs == MPX_OK) rs = replay_gradient(e, cd, *fg, *plan, grad_angles, &done);
+            free_plan(e, own);
+            if (rs != MPX_OK) return rs;
+        }
+        if (done) {
+            if (nf > 0 && A.final_coef != nullptr)
+                MPX_CUDA(cudaMemcpyAsync(e->st.coef, A.final_coef, nf * sizeof(double), cudaMemcpyDeviceToDevice, e->stream));
+            Counters c{};
+            c.n = nf;
+            c.n0 = nf;
+            c.stall = kNoStall;
+            MPX_CUDA(cudaMemcpyAsync(e->d_cnt, &c, sizeof(Counters), cudaMemcpyHostToDevice, e->stream));
+            MPX_CUDA(cudaStreamSynchronize(e->stream));
+            return MPX_OK;
+        }
+    }
     // per-step bases of the tape (prefix sums within each segment) and store sizes after each step
     std::vector<uint64_t> u_base(L), p_base(L), n_next(L);
     uint64_t u_max = 1, p_max = 1;
@@ -1873,6 +2065,7 @@ mpx_status recorded_view(mpx_engine *eng, FrozenGraph &v) {
 
 void free_graph(mpx_engine *e) {
     FrozenGraph &g = e->fg;
+    free_plan(e, g.plan);
     for (void *p : {static_cast<void *>(g.src), static_cast<void *>(g.tgt), static_cast<void *>(g.code),
                     static_cast<void *>(g.p_begin), static_cast<void *>(g.p_count), static_cast<void *>(g.w_anti),
                     static_cast<void *>(g.done), static_cast<void *>(g.last), static_cast<void *>(g.longb)})
@@ -2172,10 +2365,25 @@ mpx_status frozen_forward(mpx_engine *eng, const CircuitDev &cd, uint64_t segmen
     free_adjoint(e);
     mpx_status s0 = frozen_start(e);
     if (s0 != MPX_OK) return s0;
+    uint8_t *mark = nullptr;
+    const ReplayPlan *plan = segment_gates == 0 ? graph_plan(e, cd, g) : nullptr;
+    if (plan != nullptr && dev_alloc(e, reinterpret_cast<void **>(&mark), std::max<uint64_t>(nf, 4)) != cudaSuccess) {
+        cudaGetLastError();
+        plan = nullptr;
+    }
+    if (plan != nullptr) {
+        MPX_CUDA(cudaMemsetAsync(mark, 0, std::max<uint64_t>(nf, 4), e->stream));
+        const ReplayLaunch a = replay_launch(e, cd, g);
+        for (uint32_t w = 0; w < plan->windows; ++w)
+            MPX_CUDA(replay_forward(a, *plan, w, w + 1 < plan->windows ? g.n0[static_cast<uint64_t>(w + 1) * plan->gates] : nf,
+                                    mark, nullptr, nullptr, nullptr));
+        e->launches += 2 * plan->windows;
+        dev_free(e, mark);
+    }
     const Frozen fz = g.view();
     const FrozenFn run = pick_frozen<false>(e->W);
     const uint64_t K = segment_gates == 0 ? std::max<uint64_t>(L, 1) : segment_gates;
-    for (uint64_t st = 0; st < L; ++st) {
+    for (uint64_t st = 0; st < L && plan == nullptr; ++st) {
         if (segment_gates > 0 && st % K == 0) {
             const uint64_t n = g.n0[st];
             double *ck = nullptr;
@@ -2187,7 +2395,7 @@ mpx_status frozen_forward(mpx_engine *eng, const CircuitDev &cd, uint64_t segmen
         }
         run(e, cd.d_desc, fz, static_cast<uint32_t>(L - 1 - st), static_cast<uint32_t>(st), g.n0[st], g.done, Tape{});
     }
-    e->launches += 2 * L;
+    e->launches += plan == nullptr ? 2 * L : 0;
     MPX_CUDA(cudaGetLastError());
     Counters c{};
     c.n = nf;
@@ -2734,9 +2942,14 @@ mpx_status mpx_adjoint_backward(mpx_engine *e, const mpx_circuit *c, double *gra
     if (c->n == 0) return MPX_OK;
     if (e->adj.log_ok) {
         // the forward pass logged everything: the reverse sweep alone
-        const mpx_status s = adjoint_backward_logged(e, *c, grad_angles);
-        if (s == MPX_OK) schr_grad_to_layers(e, grad_angles, c->n);
-        return s;
+        FrozenGraph logged;
+        mpx_status s = recorded_view(e, logged);
+        if (s != MPX_OK) return s;
+        bool done = false;
+        s = adjoint_backward_logged(e, *c, logged, grad_angles, &done);
+        dev_free(e, logged.p_count);
+        if (s == MPX_OK && done) schr_grad_to_layers(e, grad_angles, c->n);
+        if (s != MPX_OK || done) return s;
     }
     if (!e->adj.rec_ok) {
         // the streaming replay runs with the forward pass's only_rotate_len_k

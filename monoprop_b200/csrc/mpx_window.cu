@@ -1,5 +1,8 @@
 // mpx_window.cu -- launchers of the window kernels (mpx_window.cuh), one variant per key width, basis and
 // basis_change. A translation unit of its own: it compiles beside the engine's.
+#include <algorithm>
+
+#include "mpx_replay.cuh"
 #include "mpx_window.cuh"
 
 namespace mpx {
@@ -63,6 +66,73 @@ cudaError_t window_gates(const WindowLaunch &a, uint32_t hi) {
     case 7: return gates_w<7>(a, hi);
     default: return gates_w<8>(a, hi);
     }
+}
+
+// ----- replay of a frozen structure (mpx_replay.cuh) -----
+
+namespace {
+unsigned pair_blocks(uint64_t count) { return static_cast<unsigned>(std::max<uint64_t>(1, std::min<uint64_t>((count + 255) / 256, 2368))); }
+
+template <int W>
+void count_w(const ReplayLaunch &a, const ReplayPlan &p, const ReplaySort &s, uint32_t window, const uint32_t *src,
+             const uint64_t *p_begin, const unsigned long long *p_count, uint64_t first, uint64_t count) {
+    k_replay_count<W><<<pair_blocks(count), 256, 0, a.stream>>>(a.st.keys, p, s, window, a.L, src, p_begin, p_count, first, count);
+}
+}  // namespace
+
+cudaError_t replay_tables(const ReplayLaunch &a, const ReplayPlan &p, const ReplaySort &s) {
+    k_replay_tables<<<p.windows, 256, 0, a.stream>>>(a.desc, a.L, a.W, p, s.tables);
+    return cudaGetLastError();
+}
+
+cudaError_t replay_count(const ReplayLaunch &a, const ReplayPlan &p, const ReplaySort &s, uint32_t window,
+                         const uint32_t *src, const uint64_t *p_begin, const unsigned long long *p_count, uint64_t first,
+                         uint64_t count) {
+    if (count == 0) return cudaSuccess;
+    switch (a.W) {
+    case 1: count_w<1>(a, p, s, window, src, p_begin, p_count, first, count); break;
+    case 2: count_w<2>(a, p, s, window, src, p_begin, p_count, first, count); break;
+    case 3: count_w<3>(a, p, s, window, src, p_begin, p_count, first, count); break;
+    case 4: count_w<4>(a, p, s, window, src, p_begin, p_count, first, count); break;
+    case 5: count_w<5>(a, p, s, window, src, p_begin, p_count, first, count); break;
+    case 6: count_w<6>(a, p, s, window, src, p_begin, p_count, first, count); break;
+    case 7: count_w<7>(a, p, s, window, src, p_begin, p_count, first, count); break;
+    default: count_w<8>(a, p, s, window, src, p_begin, p_count, first, count); break;
+    }
+    return cudaGetLastError();
+}
+
+cudaError_t replay_prefix(const ReplayLaunch &a, const ReplayPlan &p, const ReplaySort &s) {
+    k_replay_prefix<<<p.windows, 1024, 0, a.stream>>>(p, s);
+    return cudaGetLastError();
+}
+
+cudaError_t replay_scatter(const ReplayLaunch &a, const ReplayPlan &p, const ReplaySort &s, uint32_t window,
+                           const uint32_t *src, const uint32_t *tgt, const int8_t *code, const double *in_vs,
+                           const double *in_vt, double *vs, double *vt, const uint64_t *p_begin,
+                           const unsigned long long *p_count, uint64_t first, uint64_t count) {
+    if (count == 0) return cudaSuccess;
+    k_replay_scatter<<<pair_blocks(count), 256, 0, a.stream>>>(p, s, window, a.L, src, tgt, code, in_vs, in_vt, vs, vt,
+                                                               p_begin, p_count, first, count);
+    return cudaGetLastError();
+}
+
+cudaError_t replay_forward(const ReplayLaunch &a, const ReplayPlan &p, uint32_t window, uint64_t n_end, uint8_t *last,
+                           double *vs, double *vt, double *ck) {
+    const uint32_t lo = window * p.gates, n = std::min(p.gates, a.L - lo);
+    k_replay_pairs<<<p.sectors, kSectorThreads, 0, a.stream>>>(a.st.coef, last, a.longb, p, window, a.desc, a.L, vs, vt);
+    k_replay_close<<<a.blocks, kCloseWarps * 32, 0, a.stream>>>(a.st, 64u * a.W, a.longb, last, a.desc, a.L, lo, n,
+                                                                n_end, ck);
+    return cudaGetLastError();
+}
+
+cudaError_t replay_reverse(const ReplayLaunch &a, const ReplayPlan &p, uint32_t window, uint64_t n_start, double *lam,
+                           uint8_t *event, const double *vs, const double *vt, const double *ck, double *grad) {
+    const uint32_t lo = window * p.gates, n = std::min(p.gates, a.L - lo);
+    k_reverse_pairs<<<p.sectors, kSectorThreads, 0, a.stream>>>(lam, event, a.longb, p, window, a.desc, a.L, vs, vt, grad);
+    k_reverse_close<<<a.blocks, kCloseWarps * 32, 0, a.stream>>>(a.st, 64u * a.W, a.longb, lam, event, ck, a.desc, a.L, lo, n,
+                                                                 n_start, grad);
+    return cudaGetLastError();
 }
 
 }  // namespace mpx

@@ -70,8 +70,7 @@ struct TableWork {
     uint64_t odd;
 };
 __device__ __forceinline__ void window_tables(const GateDesc *__restrict__ gates, uint32_t L, uint32_t lo, int K, int W,
-                                              WindowCtl *ctl, TableWork &s) {
-    WindowTables &t = ctl->tables;
+                                              WindowTables &t, uint64_t *comm, TableWork &s) {
     const int tid = static_cast<int>(threadIdx.x), T = static_cast<int>(blockDim.x);
     for (int k = tid; k < kWindow * W; k += T) {
         const int j = k / W, w = k % W;
@@ -101,7 +100,7 @@ __device__ __forceinline__ void window_tables(const GateDesc *__restrict__ gates
             pop += __popcll(s.rows[tid][w]);
             for (uint64_t x = s.rows[tid][w]; x != 0; x &= x - 1) mask ^= s.mask[64 * w + __ffsll(static_cast<long long>(x)) - 1];
         }
-        ctl->comm[tid] = (pop & 1) ? mask ^ s.odd : mask;
+        comm[tid] = (pop & 1) ? mask ^ s.odd : mask;
     }
     __syncthreads();
     const int r = tid % kWindow; // row r, words tid / kWindow, ...
@@ -139,6 +138,21 @@ __device__ __forceinline__ void window_tables(const GateDesc *__restrict__ gates
 constexpr int kCloseWarps = 8;
 constexpr int kCloseWords = 8;  // column words (256 terms, one 32-byte sector per column) per warp and turn
 constexpr int kClosePitch = 9;  // padded row of the anticommutation words (bank conflicts)
+
+// Word j of a gate's columns after the first four, and of the parity column for odd generators.
+__device__ __forceinline__ uint32_t more_columns(const GateDesc &gd, const Store &st, uint32_t parity_col, uint32_t j) {
+    uint32_t a = 0;
+    if (gd.n_fold <= kMaxFoldCols) {
+        for (int f = 4; f < gd.n_fold; ++f) a ^= st.cols[static_cast<uint64_t>(gd.fold_cols[f]) * st.cstride + j];
+    }
+    else {
+        for (uint32_t wd = 0; wd < parity_col / 64; ++wd)
+            for (uint64_t x = gd.fold[wd]; x != 0; x &= x - 1)
+                a ^= st.cols[(64ull * wd + __ffsll(static_cast<long long>(x)) - 1) * st.cstride + j];
+    }
+    if (gd.g_odd != 0) a ^= st.cols[static_cast<uint64_t>(parity_col) * st.cstride + j];
+    return a;
+}
 
 // Applies the pending window (ctl) to its passive terms and collects the candidates of the next window, of at
 // most kWindow gates from cnt->step on and before hi. Bound by memory: 16 bytes of coefficient per term and the columns of
@@ -185,8 +199,8 @@ __global__ void __launch_bounds__(kCloseWarps * 32, 4)
     if (done == 0 && !next) return;
     if (blockIdx.x == gridDim.x - 1) { // the last block prepares the next window's tables while the others stream
         if (next)
-            window_tables(gates, L, next_lo, static_cast<int>(next_hi - next_lo), static_cast<int>(parity_col / 64), ctl,
-                          *reinterpret_cast<TableWork *>(&s_word[0][0]));
+            window_tables(gates, L, next_lo, static_cast<int>(next_hi - next_lo), static_cast<int>(parity_col / 64),
+                          ctl->tables, ctl->comm, *reinterpret_cast<TableWork *>(&s_word[0][0]));
         return;
     }
     const uint32_t blocks = gridDim.x - 1;
@@ -243,17 +257,7 @@ __global__ void __launch_bounds__(kCloseWarps * 32, 4)
                         }
                         anti[h] = v[0] ^ v[1] ^ v[2] ^ v[3];
                         if (s_more[g]) {
-                            const GateDesc &gd = gates[L - 1 - (lo + g)];
-                            if (gd.n_fold <= kMaxFoldCols) {
-                                for (int f = 4; f < gd.n_fold; ++f)
-                                    anti[h] ^= st.cols[static_cast<uint64_t>(gd.fold_cols[f]) * st.cstride + j];
-                            }
-                            else {
-                                for (uint32_t wd = 0; wd < parity_col / 64; ++wd)
-                                    for (uint64_t x = gd.fold[wd]; x != 0; x &= x - 1)
-                                        anti[h] ^= st.cols[(64ull * wd + __ffsll(static_cast<long long>(x)) - 1) * st.cstride + j];
-                            }
-                            if (gd.g_odd != 0) anti[h] ^= st.cols[static_cast<uint64_t>(parity_col) * st.cstride + j];
+                            anti[h] ^= more_columns(gates[L - 1 - (lo + g)], st, parity_col, j);
                         }
                         if (j == nw_start - 1) anti[h] &= tail;
                     }
