@@ -503,29 +503,34 @@ void launch_replay(mpx_engine *e, const GateDesc *d_desc, uint32_t gate, uint32_
 constexpr uint32_t kSmallCap[5] = {0, 8192, 6144, 4096, 4096};
 constexpr uint32_t kSmallTableBits[5] = {0, 14, 14, 13, 13};
 
-template <int W, int B>
+template <int W, int B, bool MAPPED>
 cudaError_t launch_small(mpx_engine *e, const GateDesc *d_desc, uint32_t L, uint32_t lo, uint32_t hi) {
     const uint32_t cap = kSmallCap[W], tbits = kSmallTableBits[W];
     const size_t bytes = small_smem_bytes(W, cap, tbits);
     static bool configured = false; // per instantiation; the attribute is per function
     if (!configured) {
-        const cudaError_t ce = cudaFuncSetAttribute(k_small<W, B>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        const cudaError_t ce = cudaFuncSetAttribute(k_small<W, B, MAPPED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                     static_cast<int>(bytes));
         if (ce != cudaSuccess) return ce;
         configured = true;
     }
-    k_small<W, B><<<1, kSmallThreads, bytes, e->stream>>>(e->st, e->d_cnt, d_desc, L, lo, hi, e->tr, e->d_stats, cap,
+    k_small<W, B, MAPPED><<<1, kSmallThreads, bytes, e->stream>>>(e->st, e->d_cnt, d_desc, L, lo, hi, e->tr, e->d_stats, cap,
                                                          tbits);
     return cudaGetLastError();
 }
 
 using SmallFn = cudaError_t (*)(mpx_engine *, const GateDesc *, uint32_t, uint32_t, uint32_t);
-SmallFn pick_small(int W, int basis) {
+template <int W>
+SmallFn small_fn(int basis, bool mapped) {
+    if (basis == 1) return &launch_small<W, 1, false>;
+    return mapped ? &launch_small<W, 0, true> : &launch_small<W, 0, false>;
+}
+SmallFn pick_small(int W, int basis, bool mapped) {
     switch (W) {
-    case 1: return basis == 1 ? &launch_small<1, 1> : &launch_small<1, 0>;
-    case 2: return basis == 1 ? &launch_small<2, 1> : &launch_small<2, 0>;
-    case 3: return basis == 1 ? &launch_small<3, 1> : &launch_small<3, 0>;
-    case 4: return basis == 1 ? &launch_small<4, 1> : &launch_small<4, 0>;
+    case 1: return small_fn<1>(basis, mapped);
+    case 2: return small_fn<2>(basis, mapped);
+    case 3: return small_fn<3>(basis, mapped);
+    case 4: return small_fn<4>(basis, mapped);
     default: return nullptr;
     }
 }
@@ -1185,7 +1190,7 @@ mpx_status run_range(mpx_engine *eng, const CircuitDev &cd, uint64_t lo, uint64_
     uint64_t pending_slot = 0;
     // Small store: run gates in one shared-memory block until the store outgrows it (or the range ends).
 
-    if (e->small_path && e->W <= 4 && !e->profile && !cd.any_cos_zero && !e->tr.has_len_k && e->tr.basis_rows == nullptr &&
+    if (e->small_path && e->W <= 4 && !e->profile && !cd.any_cos_zero && !e->tr.has_len_k &&
         e->fwd_tape.w_anti == nullptr &&
         hi - lo >= 8) {
         MPX_CUDA(cudaMemcpyAsync(e->h_cnt, e->d_cnt, sizeof(Counters), cudaMemcpyDeviceToHost, e->stream));
@@ -1197,7 +1202,7 @@ mpx_status run_range(mpx_engine *eng, const CircuitDev &cd, uint64_t lo, uint64_
                 s = alloc_store(e, 2 * cap_small, n_now);
                 if (s != MPX_OK) return s;
             }
-            MPX_CUDA(pick_small(e->W, e->cfg.basis)(e, cd.d_desc, static_cast<uint32_t>(L), static_cast<uint32_t>(lo),
+            MPX_CUDA(pick_small(e->W, e->cfg.basis, e->tr.basis_rows != nullptr)(e, cd.d_desc, static_cast<uint32_t>(L), static_cast<uint32_t>(lo),
                                                    static_cast<uint32_t>(hi)));
             e->launches += 1;
             MPX_CUDA(cudaMemcpyAsync(e->h_cnt, e->d_cnt, sizeof(Counters), cudaMemcpyDeviceToHost, e->stream));
