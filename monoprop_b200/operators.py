@@ -19,6 +19,8 @@ from collections.abc import Mapping, Sequence
 import numpy as np
 
 _PAULI_LETTERS = frozenset("IXYZ")
+#: np.real_if_close's bound on the imaginary part of a double-precision complex number (100 eps)
+_REAL_IF_CLOSE = 100 * np.finfo(np.float64).eps
 
 
 def _check_size(value, name: str) -> int:
@@ -179,13 +181,19 @@ class Pauli:
     @classmethod
     def from_slots(cls, slots: Sequence[int]) -> Pauli:
         """Inverse of :meth:`slots`: (2q only) X, (2q+1 only) Y, (both) Z."""
-        present = set(int(s) for s in slots)
-        letters, qubits = [], []
-        for q in sorted({s // 2 for s in present}):
-            u, v = 2 * q in present, 2 * q + 1 in present
-            letters.append("X" if u and not v else ("Y" if v and not u else "Z"))
-            qubits.append(q)
-        return cls("".join(letters), tuple(qubits))
+        letters, qubits = "", []
+        for s in sorted({int(s) for s in slots}):
+            q = s >> 1
+            if qubits and qubits[-1] == q:  # the even slot came before: both are set
+                letters = letters[:-1] + "Z"
+            else:
+                letters += "Y" if s & 1 else "X"
+                qubits.append(q)
+        if qubits and qubits[0] < 0:
+            return cls(letters, qubits)  # refused there
+        out = cls.__new__(cls)  # letters and qubits are valid, distinct and sorted: nothing left to check
+        out.qubits, out.string = tuple(qubits), letters
+        return out
 
     def __eq__(self, other) -> bool:
         return isinstance(other, Pauli) and (self.string, self.qubits) == (other.string, other.qubits)
@@ -204,10 +212,16 @@ class PauliOperator:
         acc: dict[Pauli, float] = defaultdict(float)
         for key, c in terms.items():
             p = key if isinstance(key, Pauli) else Pauli(key)
-            v = np.real_if_close(c)
-            if np.iscomplexobj(v):
-                raise ValueError("Operator has complex terms")
-            acc[p] += float(v)
+            if type(c) is complex and abs(c.imag) < _REAL_IF_CLOSE:
+                v = c.real
+            elif type(c) is float:
+                v = c
+            else:
+                v = np.real_if_close(c)
+                if np.iscomplexobj(v):
+                    raise ValueError("Operator has complex terms")
+                v = float(v)
+            acc[p] += v
         self.terms: dict[Pauli, float] = dict(acc)
         self.num_qubits = _check_size(num_qubits, "num_qubits")
         for p in self.terms:
