@@ -143,7 +143,8 @@ __device__ __forceinline__ double pair_phase(int8_t code) { return static_cast<d
 
 // The pairs of one window, one sector per block. last[i]: the gates of the window already applied to term i.
 // Bound by latency: per gate the two coefficients' loads and a block barrier; the next gate's pairs are loaded
-// before the barrier.
+// before the barrier. (Pairs two gates ahead with their coefficients prefetched to L2 one gate ahead were slower:
+// 6x6 Hubbard loop 3.23 -> 3.78 ms.)
 __global__ void __launch_bounds__(kSectorThreads, kSectorsPerSM)
     k_replay_pairs(double *__restrict__ coef, uint8_t *__restrict__ last, const uint32_t *__restrict__ longb, ReplayPlan p, uint32_t window,
                    const GateDesc *__restrict__ gates, uint32_t L, double *__restrict__ vs_log, double *__restrict__ vt_log) {
@@ -234,10 +235,10 @@ __device__ __forceinline__ void dense_words(uint32_t *sw, const DenseShared &s, 
     const uint32_t j = j0 + w, nw = static_cast<uint32_t>((n_terms + 31) >> 5);
     uint32_t kept = j < nw && longb != nullptr ? ~longb[j] : 0xFFFFFFFFu;
     if (j == nw - 1 && (n_terms & 31) != 0) kept &= (1u << (n_terms & 31)) - 1u;
-    for (uint32_t g0 = 0; g0 < n; g0 += 8) {
-        uint32_t anti[2] = {0, 0};
+    for (uint32_t g0 = 0; g0 < n; g0 += 16) {
+        uint32_t anti[4] = {0, 0, 0, 0};
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
+        for (int h = 0; h < 4; ++h) {
             const uint32_t g = g0 + 4 * h + (lane >> 3);
             if (g >= n || j >= nw) continue;
             uint32_t v[4];
@@ -251,7 +252,7 @@ __device__ __forceinline__ void dense_words(uint32_t *sw, const DenseShared &s, 
             anti[h] &= kept;
         }
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
+        for (int h = 0; h < 4; ++h) {
             const uint32_t g = g0 + 4 * h + (lane >> 3);
             if (g < kWindow) sw[g * kClosePitch + w] = anti[h];
         }

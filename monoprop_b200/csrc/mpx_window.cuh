@@ -242,11 +242,11 @@ __global__ void __launch_bounds__(kCloseWarps * 32, 4)
             if (lane < kCloseWords && j0 + lane < nw_start) actw = ws.act[j0 + lane];
             const int w = lane & 7;
             const uint32_t j = j0 + w;
-            for (int g0 = 0; g0 < static_cast<int>(done); g0 += 8) {
-                // two gates per lane and turn, so that up to 16 column loads are in flight
-                uint32_t anti[2] = {0, 0};
+            for (int g0 = 0; g0 < static_cast<int>(done); g0 += 16) {
+                // four gates per lane and turn, up to 16 column loads in flight (two gates: 4 % longer)
+                uint32_t anti[4] = {0, 0, 0, 0};
 #pragma unroll
-                for (int h = 0; h < 2; ++h) {
+                for (int h = 0; h < 4; ++h) {
                     const int g = g0 + 4 * h + (lane >> 3);
                     if (g < static_cast<int>(done) && j < nw_start) {
                         uint32_t v[4];
@@ -263,7 +263,7 @@ __global__ void __launch_bounds__(kCloseWarps * 32, 4)
                     }
                 }
 #pragma unroll
-                for (int h = 0; h < 2; ++h) {
+                for (int h = 0; h < 4; ++h) {
                     const int g = g0 + 4 * h + (lane >> 3);
                     if (g < kWindow) sw[g * kClosePitch + w] = anti[h];
                 }
