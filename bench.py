@@ -429,29 +429,21 @@ def main() -> None:
     h2d = int(gw.nbytes + ang.nbytes + keys.nbytes + coefs.nbytes)
 
     peak, peak_kind = _peaks()
-    sweep_avg_s = statistics.mean(sweep_ms) * 1e-3
-    achieved = sweep_bytes / sweep_avg_s / 1e9
-    roofline = {"bound": "hbm", "kernel": "k_sweep", "achieved": achieved, "peak": peak, "unit": "GB/s",
+    # What the path cannot do without, against the whole step: per gate the anticommuting coefficients read and
+    # written and the appended rows written (the store exceeds L2). sweep_bytes is what a gate-by-gate sweep over
+    # the bit-columns moves for the same circuit.
+    floor_bytes = float((16 * anti + (8 * W + 8) * app).sum())
+    achieved = floor_bytes / (ms_per_step * 1e-3) / 1e9
+    roofline = {"bound": "hbm", "kernel": "window kernels (whole step)", "achieved": achieved, "peak": peak, "unit": "GB/s",
                 "frac": achieved / peak, "peak_source": f"{peak_kind} hbm_gbs",
-                "traffic": None, "algorithmic_bytes_per_launch": sweep_bytes / wl.n_layers,
-                "avg_launch_us": sweep_avg_s / wl.n_layers * 1e6,
-                "kernel_ms_per_step": {"k_sweep": statistics.mean(sweep_ms), "k_resolve": statistics.mean(resolve_ms)},
+                "traffic": None, "algorithmic_bytes_per_step": floor_bytes, "gate_by_gate_bytes_per_step": sweep_bytes,
+                "kernel_ms_per_step": {"dense passes": statistics.mean(sweep_ms),
+                                       "lists, gates, commit": statistics.mean(resolve_ms)},
                 "path_bytes_per_step": path_bytes,
-                # the sweep's binding resource: random 32-byte DRAM sectors (each anticommuting coefficient is
-                # read and written once, each emitted term's key row read), per second of sweep time
-                "random_sectors_per_s": float((2 * anti + np.ceil(W / 4) * emitted).sum()) / (statistics.mean(sweep_ms) * 1e-3),
                 # per step: anticommuting terms (cos-scaled), emitted sine branches, appended partners
                 "anticommuting_per_step": int(anti.sum()), "emitted_per_step": int(emitted.sum()),
                 "appended_per_step": int(app.sum()),
                 "path_frac": path_bytes / (ms_per_step * 1e-3) / 1e9 / peak}
-    # DRAM bytes per launch: the ncu-measured traffic/algorithmic ratio of the sweep (captured on this
-    # circuit itself at 8.0e6 terms, `--regime-case`), scaled to the average launch's algorithmic bytes.
-    traffic_file = os.path.join(ROOT, "profiles", "k_sweep_traffic.json")
-    if os.path.exists(traffic_file):
-        with open(traffic_file) as f:
-            ratio = json.load(f)["traffic_over_algorithmic"]
-        roofline["traffic"] = ratio * sweep_bytes / wl.n_layers
-        roofline["traffic_source"] = "ncu ratio from profiles/k_sweep_traffic.json x algorithmic bytes"
 
     if dist is not None:
         dist.barrier()

@@ -1445,10 +1445,12 @@ void free_adjoint(mpx_engine *e) {
 }
 
 // Gates per replay window. Sectors stay balanced while the rank of the window's generators is well below the
-// number of key bits in use (2 per mode): on the 5x10 lattice 64 gates leave a few hundred cosets (busiest block
-// 8 times the mean), 25 leave it at 1.3 times; on the 6x6 Hubbard lattice 64 give 2.8, 36 give 1.6.
+// number of key bits in use (2 per mode; on the 5x10 lattice 64 gates leave a few hundred cosets, busiest block 8
+// times the mean, 32 leave it at 1.2-1.4), and longer windows make fewer dense passes. Measured per 8 modes: 4, 5
+// and 6 gates give 17.9, 16.8 and 17.2 ms for the reverse sweep of the 50-qubit gradient (8 layers) and 3.23, 2.87
+// and 2.82 ms per call of the 6x6 Hubbard loop.
 uint32_t replay_window(const mpx_engine *e) {
-    return static_cast<uint32_t>(std::min<int>(kWindow, std::max(8, e->cfg.num_modes / 2)));
+    return static_cast<uint32_t>(std::min<int>(kWindow, std::max(8, 5 * e->cfg.num_modes / 8)));
 }
 
 // Forward pass for the gradient: resets the store to the initial operator, propagates the circuit
