@@ -1678,9 +1678,10 @@ mpx_status build_plan(mpx_engine *eng, const CircuitDev &cd, const FrozenGraph &
 }
 
 // The plan of the engine's graph, built at its first replay; nullptr when the graph replays gate by gate (see
-// build_plan) and when a gate has cos == 0 (kappa needs the quotient).
+// build_plan), when a gate has cos == 0 (kappa needs the quotient) and while the graph is pared: a pared term keeps
+// the value of its last relevant step, and the plan's lazy cos factors know no such step.
 const ReplayPlan *graph_plan(mpx_engine *e, const CircuitDev &cd, FrozenGraph &g) {
-    if (!e->window_path || cd.any_cos_zero || g.no_plan) return nullptr;
+    if (!e->window_path || cd.any_cos_zero || g.no_plan || g.pared) return nullptr;
     if (g.plan.windows == 0) {
         if (build_plan(e, cd, g, nullptr, nullptr, nullptr, nullptr, g.plan) != MPX_OK || g.plan.windows == 0) {
             g.no_plan = true;
