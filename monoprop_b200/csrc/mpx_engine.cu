@@ -44,6 +44,7 @@ struct mpx_circuit {
     int W = 1;
     int device = 0;
     bool any_cos_zero = false; // some gate has cos(2 angle) == 0 exactly (needs the pre-gate copy `aux`)
+    int rank = 0; // of the generators as bit vectors (a resident circuit's; see replay_window)
 };
 using CircuitDev = mpx_circuit;
 
@@ -1444,13 +1445,41 @@ void free_adjoint(mpx_engine *e) {
     e->fwd_tape = Tape{};
 }
 
-// Gates per replay window. Sectors stay balanced while the rank of the window's generators is well below the
-// number of key bits in use (2 per mode; on the 5x10 lattice 64 gates leave a few hundred cosets, busiest block 8
-// times the mean, 32 leave it at 1.2-1.4), and longer windows make fewer dense passes. Measured per 8 modes: 4, 5
-// and 6 gates give 17.9, 16.8 and 17.2 ms for the reverse sweep of the 50-qubit gradient (8 layers) and 3.23, 2.87
-// and 2.82 ms per call of the 6x6 Hubbard loop.
-uint32_t replay_window(const mpx_engine *e) {
-    return static_cast<uint32_t>(std::min<int>(kWindow, std::max(8, 5 * e->cfg.num_modes / 8)));
+// Rank over GF(2) of n keys of W words.
+int generator_rank(const uint64_t *words, uint64_t n, int W) {
+    std::vector<int> row_of(64 * W, -1); // basis row that starts at a bit
+    std::vector<uint64_t> rows;
+    int rank = 0;
+    std::vector<uint64_t> v(W);
+    for (uint64_t k = 0; k < n; ++k) {
+        std::copy(words + k * W, words + (k + 1) * W, v.begin());
+        for (int w = 0; w < W; ++w) {
+            while (v[w] != 0) {
+                const int bit = 64 * w + __builtin_ctzll(v[w]);
+                if (row_of[bit] < 0) {
+                    row_of[bit] = rank++;
+                    rows.insert(rows.end(), v.begin(), v.end());
+                    v[w] = 0;
+                    w = W;
+                    break;
+                }
+                const uint64_t *r = &rows[static_cast<size_t>(row_of[bit]) * W];
+                for (int i = w; i < W; ++i) v[i] ^= r[i];
+            }
+        }
+    }
+    return rank;
+}
+
+// Gates per replay window. A window leaves 2^(rank of the circuit's generators - rank of its own) cosets of every
+// class of terms that the circuit connects, and sectors stay balanced while those are many; longer windows make
+// fewer dense passes. (On the 5x10 lattice, rank 99, 64 gates leave a few hundred occupied cosets, busiest block 8 times the mean,
+// 32 leave it at 1.2-1.4.) Measured per 16 of the rank: 4, 5 and 6 gates give 17.9, 16.8 and 17.2 ms for the reverse
+// sweep of the 50-qubit gradient (8 layers) and 3.23, 2.87 and 2.82 ms per call of the 6x6 Hubbard loop. The rank and
+// not the number of modes: 150 gates on 10 of 161 modes are one coset per 64 gates, and one block replayed 1e6
+// terms (744 ms per gradient, 5.4 ms gate by gate).
+uint32_t replay_window(const CircuitDev &cd) {
+    return static_cast<uint32_t>(std::min<int>(kWindow, std::max(8, (5 * cd.rank + 15) / 16)));
 }
 
 // Forward pass for the gradient: resets the store to the initial operator, propagates the circuit
@@ -1509,7 +1538,7 @@ mpx_status adjoint_forward(mpx_engine *eng, const CircuitDev &cd, uint64_t segme
             if (ce == cudaSuccess) {
                 e->fwd_tape.r_vs = A.r_vs;
                 e->fwd_tape.r_vt = A.r_vt;
-                K = replay_window(e);
+                K = replay_window(cd);
             }
             else {
                 cudaGetLastError(); // no room after all: the backward pass replays segments
@@ -1567,7 +1596,7 @@ mpx_status adjoint_forward(mpx_engine *eng, const CircuitDev &cd, uint64_t segme
     for (uint64_t st = 0; st < L; ++st) undo += e->adj.stats[4 * st + 1];
     if (log_all) e->undo_hint = undo;
     e->ck_hint = 0;
-    const uint64_t window = replay_window(e);
+    const uint64_t window = replay_window(cd);
     for (uint64_t st = 0; st < L; st += window) e->ck_hint += e->adj.stats[4 * st];
     return MPX_OK;
 }
@@ -1619,7 +1648,7 @@ mpx_status build_plan(mpx_engine *eng, const CircuitDev &cd, const FrozenGraph &
     MPX_CUDA(cudaStreamSynchronize(e->stream));
     // pairs of every window, and its range of the log (with the places a replayed build's log leaves empty)
     uint64_t total = 0;
-    const uint32_t K = replay_window(e), n_win = static_cast<uint32_t>((L + K - 1) / K);
+    const uint32_t K = replay_window(cd), n_win = static_cast<uint32_t>((L + K - 1) / K);
     std::vector<uint64_t> range(n_win, 0);
     std::vector<uint32_t> base(n_win, 0);
     for (uint64_t st = 0; st < L; ++st) {
@@ -2671,6 +2700,7 @@ mpx_status mpx_circuit_upload(mpx_engine *e, const uint64_t *gen_words, const do
     if (c == nullptr) return fail(eng, MPX_ERR_NOMEM, "host allocation failed");
     mpx_status s = upload_circuit(e, gen_words, angles, n_layers, *c);
     c->persistent = true;
+    if (s == MPX_OK) c->rank = generator_rank(gen_words, n_layers, e->W);
     if (s != MPX_OK) {
         mpx_circuit_destroy(c);
         return s;

@@ -1,0 +1,51 @@
+"""When a frozen structure replays in windows (csrc/mpx_replay.cuh) and when gate by gate.
+
+Both replays give the same numbers (test_gpu_replay.py); these tests look at what a call costs, in launches or, where a
+wrong choice costs a factor of a hundred, in time.
+"""
+
+import time
+
+import numpy as np
+import pytest
+
+from monoprop_b200 import _native
+from monoprop_b200 import workloads as W
+
+pytestmark = pytest.mark.gpu
+
+
+def on_few_modes(modes, used, gates, seed):
+    """Random Pauli generators on `used` of the modes: the operator fills their 4^used strings."""
+    rng = np.random.default_rng(seed)
+    pool = np.array([2 * m + h for m in rng.choice(modes, size=used, replace=False) for h in (0, 1)])
+    slots = [tuple(sorted(int(x) for x in rng.choice(pool, size=int(rng.choice([1, 2, 2, 3, 4])), replace=False)))
+             for _ in range(gates)]
+    z = 2 * (int(pool[0]) // 2)
+    return W.Workload("few", "pauli", modes, slots, np.ones(gates), np.arange(gates), rng.uniform(-0.5, 0.5, size=gates),
+                      {(z, z + 1): 1.0 + 0j}, [], 2 * modes, "support", None)
+
+
+def graph(wl):
+    eng = _native.engine_for(wl)
+    circ = eng.upload(wl.gen_words(), wl.angles())
+    eng.graph_build(circ)
+    return eng, circ
+
+
+@pytest.mark.parametrize("modes", [20, 161])
+def test_generators_on_few_modes_do_not_put_the_store_on_one_block(modes):
+    """Two segments replay gate by gate. One block for all terms takes some hundred times as long as that."""
+    wl = on_few_modes(modes, 9, 120, 1)
+    eng, circ = graph(wl)
+
+    def seconds(segment_gates):
+        eng.graph_gradient(circ, segment_gates=segment_gates)
+        t = time.perf_counter()
+        eng.graph_gradient(circ, segment_gates=segment_gates)
+        return time.perf_counter() - t
+
+    windows, gate_by_gate = seconds(0), seconds(60)
+    circ.close()
+    eng.close()
+    assert windows <= 5 * gate_by_gate
