@@ -159,7 +159,8 @@ struct mpx_engine {
     uint64_t store_gen = 0;
     uint64_t rec_hint = 0; // pair records the last recording forward pass needed (sizes the next log)
     uint64_t ck_hint = 0; // terms of all replay windows' checkpoints in the last gradient forward pass
-    uint64_t undo_hint = 0; // undo records (anticommuting terms over all gates) of the last gradient forward pass
+    uint64_t log_pays = 0; // circuit whose next gradient forward pass logs what the reverse sweep needs (0: none)
+    uint64_t unbalanced = 0; // circuit whose logged pass turned out too unbalanced to sweep in windows
     int64_t pair_log = -1; // mpx_set_pair_log: < 0 automatic, 0 off, > 0 fixed capacity
     uint64_t *d_basis = nullptr; // basis_change rows [2T][W] (tr.basis_rows points here when set)
     // Re-weighted initial operator (mpx_update_initial_operator): store indices and coefficients that
@@ -1482,6 +1483,28 @@ uint32_t replay_window(const CircuitDev &cd) {
     return static_cast<uint32_t>(std::min<int>(kWindow, std::max(8, (5 * cd.rank + 15) / 16)));
 }
 
+// Whether a gradient over a frozen structure takes less time in windows than gate by gate. Windows: 64 us for each
+// (launches and its sectors' chains of gates), 54 ps per term and dense pass, 257 ps per pair, or 33 ns per pair of
+// every window's busiest sector if those are more. Gate by gate: 12.1 us per gate, 21 ps per anticommuting term, 81 ps
+// per pair (its pairs kernel reads a log in store order, a sector's pairs are scattered over the store). Least-squares
+// fit over 33 circuits (lines, lattices, Hubbard lattices, random generators on 8 to 12 modes; 4e3 to 2.9e7 terms, 138
+// to 3360 gates), every one of them predicted within 30 %; ratios of the two from 0.2 (few of the terms are paired) to
+// 1.9 (all of them are: up to 12 qubits without truncation). At predicted ratios around 0.95 both sides measure alike,
+// so that is where a graph's replay changes over. A gradient that has logged its forward pass sweeps in windows or not
+// at all, and the log spares it the tape of a replay: it is kept up to 1.4 (20-qubit line, Schrodinger, 1.3: 10.8 ms
+// with the log, 10.1 without; 10 qubits, all terms paired, 1.7: 15.0 and 12.1 ms).
+constexpr double kReplayPays = 0.95, kLogPays = 1.4;
+struct ReplayWork {
+    uint64_t gates, window;    // of the circuit, of a window
+    double terms, anti, pairs; // over all gates
+    double busiest;            // pairs of the busiest sector, over all windows (0: not known)
+};
+bool replay_pays(const ReplayWork &r, double most) {
+    const double windows = 64.0 * static_cast<double>((r.gates + r.window - 1) / r.window) +
+                           5.4e-5 * r.terms / static_cast<double>(r.window) + std::max(2.57e-4 * r.pairs, 0.033 * r.busiest);
+    return windows <= most * (12.1 * static_cast<double>(r.gates) + 2.1e-5 * r.anti + 8.1e-5 * r.pairs);
+}
+
 // Forward pass for the gradient: resets the store to the initial operator, propagates the circuit
 // segment by segment (segment_gates gates each) and saves the coefficient array at every segment start
 // and at the end. With log_all, and when the previous gradient forward pass of this engine says how many
@@ -1524,7 +1547,7 @@ mpx_status adjoint_forward(mpx_engine *eng, const CircuitDev &cd, uint64_t segme
     // Logging everything the reverse sweep needs: both values of every pair, and a checkpoint per replay window
     // (segments of that length). Needs the size of the pair log, which the previous pass of this engine gives.
     uint64_t K = segment_gates == 0 ? std::max<uint64_t>(L, 1) : segment_gates;
-    if (log_all && e->window_path && e->fwd_tape.r_src != nullptr && e->undo_hint > 0 && !cd.any_cos_zero) {
+    if (log_all && e->window_path && e->fwd_tape.r_src != nullptr && e->log_pays == cd.id && !cd.any_cos_zero) {
         AdjointState &A = e->adj;
         const uint64_t r_cap = e->fwd_tape.r_cap;
         // the values twice (as logged, and sorted for the reverse sweep), the sorted pairs, the checkpoints; large
@@ -1591,12 +1614,15 @@ mpx_status adjoint_forward(mpx_engine *eng, const CircuitDev &cd, uint64_t segme
     MPX_CUDA(cudaStreamSynchronize(e->stream));
     e->last_gates = L;
     e->adj.circuit = &cd;
-    // undo records the circuit needs (every anticommuting term of every gate): sizes the next pass's log
-    uint64_t undo = 0;
-    for (uint64_t st = 0; st < L; ++st) undo += e->adj.stats[4 * st + 1];
-    if (log_all) e->undo_hint = undo;
-    e->ck_hint = 0;
+    // whether the next pass of this circuit logs, and the terms of its checkpoints then
     const uint64_t window = replay_window(cd);
+    ReplayWork work{L, window, 0.0, 0.0, static_cast<double>(e->adj.r_total), 0.0};
+    for (uint64_t st = 0; st < L; ++st) {
+        work.terms += static_cast<double>(e->adj.stats[4 * st]);
+        work.anti += static_cast<double>(e->adj.stats[4 * st + 1]);
+    }
+    if (log_all) e->log_pays = e->adj.r_total > 0 && cd.id != e->unbalanced && replay_pays(work, kLogPays) ? cd.id : 0;
+    e->ck_hint = 0;
     for (uint64_t st = 0; st < L; st += window) e->ck_hint += e->adj.stats[4 * st];
     return MPX_OK;
 }
@@ -1636,11 +1662,13 @@ ReplayLaunch replay_launch(const mpx_engine *e, const CircuitDev &cd, const Froz
 }
 
 // Sorts the structure's pairs into replay order. in_vs / in_vt with vs / vt: the pairs' logged values, sorted
-// along. Leaves p empty (MPX_OK) when the device has no room or the pairs have no 32-bit numbers.
+// along. Leaves p empty (MPX_OK) when windows do not pay (replay_pays, at first for balanced sectors, then for the
+// busiest as counted), the pairs have no 32-bit numbers or the device has no room (*room = false).
 mpx_status build_plan(mpx_engine *eng, const CircuitDev &cd, const FrozenGraph &g, const double *in_vs, const double *in_vt,
-                      double *vs, double *vt, ReplayPlan &p) {
+                      double *vs, double *vt, ReplayPlan &p, bool *room) {
     mpx_engine *e = eng;
     p = ReplayPlan{};
+    *room = true;
     const uint64_t L = g.L;
     if (L == 0 || g.src == nullptr) return MPX_OK;
     std::vector<uint64_t> begin(L);
@@ -1657,6 +1685,13 @@ mpx_status build_plan(mpx_engine *eng, const CircuitDev &cd, const FrozenGraph &
         range[st / K] = begin[st] + g.count[st] - begin[st / K * K];
         if (total >= 0xFFFFFFFFull) return MPX_OK;
     }
+    ReplayWork work{L, K, 0.0, 0.0, static_cast<double>(total), 0.0};
+    for (uint64_t st = 0; st < L; ++st) {
+        work.terms += static_cast<double>(g.n0[st]);
+        work.anti += static_cast<double>(g.anti[st]);
+    }
+    const double most = in_vs != nullptr ? kLogPays : kReplayPays;
+    if (!replay_pays(work, most)) return MPX_OK;
     const uint64_t places = begin[L - 1] + g.count[L - 1];
     ReplayPlan q{};
     ReplaySort so{};
@@ -1678,6 +1713,7 @@ mpx_status build_plan(mpx_engine *eng, const CircuitDev &cd, const FrozenGraph &
     A(&so.tables, n_win);
     A(&so.cursor, n_win * slots);
     A(&so.base, n_win);
+    A(&so.busiest, n_win);
     A(&so.c_mask, places);
     A(&so.c_sector, places);
     if (ce == cudaSuccess)
@@ -1688,18 +1724,29 @@ mpx_status build_plan(mpx_engine *eng, const CircuitDev &cd, const FrozenGraph &
     for (uint32_t w = 0; ce == cudaSuccess && w < n_win; ++w) 
         ce = replay_count(a, q, so, w, g.src, g.p_begin, g.p_count, begin[w * K], range[w]);
     if (ce == cudaSuccess) ce = replay_prefix(a, q, so);
-    for (uint32_t w = 0; ce == cudaSuccess && w < n_win; ++w)
+    std::vector<uint32_t> busiest(n_win, 0);
+    if (ce == cudaSuccess)
+        ce = cudaMemcpyAsync(busiest.data(), so.busiest, n_win * sizeof(uint32_t), cudaMemcpyDeviceToHost, e->stream);
+    if (ce == cudaSuccess) ce = cudaStreamSynchronize(e->stream);
+    for (const uint32_t b : busiest) work.busiest += b;
+    const bool pays = replay_pays(work, most);
+    for (uint32_t w = 0; ce == cudaSuccess && pays && w < n_win; ++w)
         ce = replay_scatter(a, q, so, w, g.src, g.tgt, g.code, in_vs, in_vt, vs, vt, g.p_begin, g.p_count, begin[w * K],
                             range[w]);
-    e->launches += 2 + 2 * n_win;
+    e->launches += 2 + (pays ? 2 : 1) * n_win;
     for (void *ptr : {static_cast<void *>(so.tables), static_cast<void *>(so.cursor), static_cast<void *>(so.base),
-                      static_cast<void *>(so.c_mask),
+                      static_cast<void *>(so.busiest), static_cast<void *>(so.c_mask),
                       static_cast<void *>(so.c_sector)})
         dev_free(e, ptr);
+    if (ce == cudaSuccess && !pays) {
+        free_plan(e, q);
+        return MPX_OK;
+    }
     if (ce != cudaSuccess) {
         free_plan(e, q);
         if (ce != cudaErrorMemoryAllocation) MPX_CUDA(ce);
         cudaGetLastError();
+        *room = false;
         return MPX_OK;
     }
     p = q;
@@ -1712,7 +1759,8 @@ mpx_status build_plan(mpx_engine *eng, const CircuitDev &cd, const FrozenGraph &
 const ReplayPlan *graph_plan(mpx_engine *e, const CircuitDev &cd, FrozenGraph &g) {
     if (!e->window_path || cd.any_cos_zero || g.no_plan || g.pared) return nullptr;
     if (g.plan.windows == 0) {
-        if (build_plan(e, cd, g, nullptr, nullptr, nullptr, nullptr, g.plan) != MPX_OK || g.plan.windows == 0) {
+        bool room = true;
+        if (build_plan(e, cd, g, nullptr, nullptr, nullptr, nullptr, g.plan, &room) != MPX_OK || g.plan.windows == 0) {
             g.no_plan = true;
             return nullptr;
         }
@@ -1799,7 +1847,7 @@ mpx_status replay_gradient(mpx_engine *eng, const CircuitDev &cd, const FrozenGr
 
 // Reverse sweep over the logs of a forward pass that logged everything (AdjointState::log_ok): the pairs are
 // sorted into replay order with their values, and the windows swept from the checkpoints at their starts. No
-// replay. *done = false (MPX_OK): no room for the sorted pairs, the caller replays the segments.
+// replay. *done = false (MPX_OK): no room for the sorted pairs, or sectors too unbalanced; the caller replays the segments.
 mpx_status adjoint_backward_logged(mpx_engine *eng, const CircuitDev &cd, const FrozenGraph &g, double *grad_angles,
                                    bool *done) {
     mpx_engine *e = eng;
@@ -1826,7 +1874,12 @@ mpx_status adjoint_backward_logged(mpx_engine *eng, const CircuitDev &cd, const 
         free_plan(e, p);
     };
     mpx_status s = MPX_OK;
-    if (ce == cudaSuccess) s = build_plan(e, cd, g, A.r_vs, A.r_vt, vs, vt, p);
+    bool room = true;
+    if (ce == cudaSuccess) s = build_plan(e, cd, g, A.r_vs, A.r_vt, vs, vt, p, &room);
+    if (ce == cudaSuccess && s == MPX_OK && p.windows == 0 && room) {
+        e->unbalanced = cd.id; // as counted, windows do not pay: the next passes do not log for them
+        e->log_pays = 0;
+    }
     if (ce != cudaSuccess || s != MPX_OK || p.windows == 0 || p.windows != A.ck_coef.size()) {
         cudaGetLastError();
         release();
@@ -1868,7 +1921,8 @@ mpx_status adjoint_backward(mpx_engine *eng, const CircuitDev &cd, double *grad_
             plan = graph_plan(e, cd, e->fg);
         }
         else if (e->window_path && !cd.any_cos_zero) {
-            const mpx_status ps = build_plan(e, cd, *fg, nullptr, nullptr, nullptr, nullptr, own);
+            bool room = true;
+            const mpx_status ps = build_plan(e, cd, *fg, nullptr, nullptr, nullptr, nullptr, own, &room);
             if (ps != MPX_OK) return ps;
             plan = own.windows != 0 ? &own : nullptr;
         }

@@ -73,9 +73,11 @@ __global__ void __launch_bounds__(256) k_replay_count(const uint64_t *__restrict
     }
 }
 
-// Counts to first pairs (exclusive prefix), one block per window; base: pairs of the windows before it.
+// Counts to first pairs (exclusive prefix), one block per window, and the busiest sector's pairs; base: pairs of the
+// windows before it.
 __global__ void __launch_bounds__(1024) k_replay_prefix(ReplayPlan p, ReplaySort so) {
-    __shared__ uint32_t s_part[32];
+    __shared__ uint32_t s_part[32], s_most;
+    if (threadIdx.x == 0) s_most = 0;
     const uint32_t n = p.sectors * p.gates;
     uint32_t *seg = p.seg + static_cast<uint64_t>(blockIdx.x) * (n + 1);
     uint32_t *cursor = so.cursor + static_cast<uint64_t>(blockIdx.x) * n;
@@ -100,6 +102,13 @@ __global__ void __launch_bounds__(1024) k_replay_prefix(ReplayPlan p, ReplaySort
         acc += c;
         if (k + 1 == n) seg[n] = acc;
     }
+    __syncthreads();
+    uint32_t most = 0;
+    for (uint32_t k = threadIdx.x; k < p.sectors; k += blockDim.x) most = max(most, seg[(k + 1) * p.gates] - seg[k * p.gates]);
+    most = __reduce_max_sync(0xFFFFFFFFu, most);
+    if (lane == 0) atomicMax(&s_most, most);
+    __syncthreads();
+    if (threadIdx.x == 0) so.busiest[blockIdx.x] = s_most;
 }
 
 __global__ void __launch_bounds__(256) k_replay_scatter(ReplayPlan p, ReplaySort so, uint32_t window, uint32_t L,

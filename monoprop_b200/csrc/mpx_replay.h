@@ -31,6 +31,7 @@ struct ReplaySort {
     WindowTables *tables;
     uint32_t *cursor;   // [windows][sectors * gates]
     uint32_t *base;     // [windows] pairs of the windows before
+    uint32_t *busiest;  // [windows] out: most pairs of one sector
     uint64_t *c_mask;
     uint16_t *c_sector;
 };

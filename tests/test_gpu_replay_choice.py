@@ -33,6 +33,24 @@ def graph(wl):
     return eng, circ
 
 
+def replay_launches(wl):
+    eng, circ = graph(wl)
+    eng.graph_expectation(circ)  # sorts the pairs, if the structure replays in windows
+    before = eng.launch_count()
+    eng.graph_expectation(circ)
+    used = eng.launch_count() - before
+    circ.close()
+    eng.close()
+    return used
+
+
+def test_dense_structures_replay_gate_by_gate_and_sparse_ones_in_windows():
+    """All of 4^10 terms paired at every gate: windows take 1.7 times as long. A lattice under lower_atol, few of whose
+    terms are paired: half as long. Gate by gate is two launches per gate, a window two launches."""
+    assert replay_launches(on_few_modes(20, 10, 150, 2)) >= 2 * 150
+    assert replay_launches(W.ising50(4)) < W.ising50(4).n_layers
+
+
 @pytest.mark.parametrize("modes", [20, 161])
 def test_generators_on_few_modes_do_not_put_the_store_on_one_block(modes):
     """Two segments replay gate by gate. One block for all terms takes some hundred times as long as that."""
