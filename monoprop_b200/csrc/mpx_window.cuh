@@ -410,9 +410,11 @@ __global__ void __launch_bounds__(256) k_window_sample(Store st, WindowScratch w
         if (s_load[0][k] != 0) atomicAdd(&ctl->load[0][k], s_load[0][k]);
 }
 
-// The window length to run, by the whole block (every block comes to the same): per gate, a sector's block takes
-// about 2.5 us plus 0.05 us per anticommuting term of the busiest sector, and a window's other launches 150 us
-// plus 20 ps per term of the store (the dense pass), spread over its gates.
+// The window length to run, by the whole block: per gate, a sector's block takes about 2.5 us plus 0.05 us per
+// anticommuting term of the busiest sector, and a window's other launches 150 us plus 20 ps per term of the store
+// (the dense pass), spread over its gates. In whole picoseconds: every block of the two kernels that ask (count, which
+// makes the masks, and scatter, which sets the window up) has to come to the same length, and floating-point sums may be contracted
+// differently in each.
 __device__ __forceinline__ int choose_length(const WindowCtl *ctl, uint32_t sectors, uint32_t most, uint64_t n, uint32_t *s_max) {
     if (threadIdx.x < kLengths) s_max[threadIdx.x] = 0;
     __syncthreads();
@@ -424,13 +426,13 @@ __device__ __forceinline__ int choose_length(const WindowCtl *ctl, uint32_t sect
         if ((threadIdx.x & 31) == 0) atomicMax(&s_max[i], m);
     }
     __syncthreads();
-    const uint32_t all = kSampleBlocks * 256 * kSamplePerThread;
-    const float scale = ctl->n_cand > all ? static_cast<float>(ctl->n_cand) / static_cast<float>(all) : 1.0f;
+    constexpr uint64_t all = kSampleBlocks * 256 * kSamplePerThread;
+    const uint64_t n_cand = ctl->n_cand;
     int best = kLengths - 1;
-    float t_best = 0.0f;
+    uint64_t t_best = 0;
     for (int i = kLengths - 1; i >= 0; --i) {
-        const float len = static_cast<float>(window_length(i, most));
-        const float t = 2.5f + (0.05f * scale * static_cast<float>(s_max[i]) + 150.0f + 2e-5f * static_cast<float>(n)) / len;
+        const uint64_t load = n_cand > all ? s_max[i] * n_cand / all : s_max[i]; // below 2^53 (2^21 sampled pairs at most)
+        const uint64_t t = 2500000 + (50000 * load + 150000000 + 20 * n) / window_length(i, most);
         if (i == kLengths - 1 || t < t_best) {
             best = i;
             t_best = t;
