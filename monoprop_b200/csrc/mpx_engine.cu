@@ -1227,9 +1227,9 @@ mpx_status run_range(mpx_engine *eng, const CircuitDev &cd, uint64_t lo, uint64_
         }
     }
     // Windows of gates over the active terms, or gate by gate: a tape, exact cos == 0 gates (their partner
-    // values need the kept pre-gate copy) and only_rotate_len_k take the per-gate kernels.
+    // values need the kept pre-gate copy), only_rotate_len_k and a few gates alone take the per-gate kernels.
     const bool windows = e->window_path && e->fwd_tape.w_anti == nullptr && !cd.any_cos_zero && !e->tr.has_len_k &&
-                         step < hi && ensure_window(e);
+                         hi - step >= kLeastGates && ensure_window(e);
     const uint64_t gen0 = e->store_gen;
     // A gradient's forward pass is not captured: its tape buffers are allocated per call, so a captured
     // range would rarely match the next call's pointers and each miss would pay a new capture.
@@ -1286,7 +1286,7 @@ mpx_status run_range(mpx_engine *eng, const CircuitDev &cd, uint64_t lo, uint64_
     for (;;) {
         bool issued = false;
         if (step == stretch && stretch < hi && !pending) {
-            if (ensure_window(e)) {
+            if (hi - step >= kLeastGates && ensure_window(e)) {
                 s = run_windows_from(false);
                 if (s != MPX_OK) return s;
             }

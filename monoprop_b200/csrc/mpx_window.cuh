@@ -410,35 +410,57 @@ __global__ void __launch_bounds__(256) k_window_sample(Store st, WindowScratch w
         if (s_load[0][k] != 0) atomicAdd(&ctl->load[0][k], s_load[0][k]);
 }
 
-// The window length to run, by the whole block: per gate, a sector's block takes about 2.5 us plus 0.05 us per
-// anticommuting term of the busiest sector, and a window's other launches 150 us plus 20 ps per term of the store
-// (the dense pass), spread over its gates. In whole picoseconds: every block of the two kernels that ask (count, which
-// makes the masks, and scatter, which sets the window up) has to come to the same length, and floating-point sums may be contracted
-// differently in each.
-__device__ __forceinline__ int choose_length(const WindowCtl *ctl, uint32_t sectors, uint32_t most, uint64_t n, uint32_t *s_max) {
-    if (threadIdx.x < kLengths) s_max[threadIdx.x] = 0;
+// The window length to run, by the whole block, or -1 when the gates take less time one by one (all in picoseconds).
+//   Windows, per gate: a sector's block takes about 2.5 us plus 0.05 us for each anticommuting term of the busiest sector
+//   (from the 33rd on, against gate by gate: the length that spreads the terms best is the better one anyhow); a window's
+//   other launches 150 us plus 20 ps per term of the store (the dense pass), spread over its gates.
+//   Gate by gate: 6.2 us for the two launches, up to 4 us for the chain of the branches, 65 ps per anticommuting
+//   active term and 1.5 ps per term (measured from 1 to 3e6 terms: 5.6 us at a few terms, 12 at 3e5 with 2e4 active and
+//   anticommuting, 33 at 1e6 with 4e5).
+// Up to 1.15 times that, windows go on (a declined try and the way back cost as much), and 0.2 ms over the gates that
+// are left in favour of windows: what a change over costs.
+// Measured on lines and lattices, windows against gate by gate: 2.0 times as long over 8 gates, 1.2 over 32, 0.8 over 64; on 8
+// to 11 qubits without truncation, where no length but the shortest is balanced, 1.2 to 2.2. In whole numbers: every
+// block of the two kernels that ask (count, which makes the masks, and scatter, which sets the window up) has to come
+// to the same length, and floating-point sums may be contracted differently in each.
+struct LengthShared {
+    uint32_t most[kLengths], sum[kLengths];
+};
+__device__ __forceinline__ int choose_length(const WindowCtl *ctl, uint32_t sectors, uint32_t most, uint64_t n, LengthShared &s) {
+    if (threadIdx.x < kLengths) s.most[threadIdx.x] = s.sum[threadIdx.x] = 0;
     __syncthreads();
 #pragma unroll
     for (int i = 0; i < kLengths; ++i) {
-        uint32_t m = 0;
-        for (uint32_t k = threadIdx.x; k < sectors; k += blockDim.x) m = max(m, ctl->load[i][k]);
+        uint32_t m = 0, t = 0;
+        for (uint32_t k = threadIdx.x; k < sectors; k += blockDim.x) {
+            m = max(m, ctl->load[i][k]);
+            t += ctl->load[i][k];
+        }
         m = __reduce_max_sync(0xFFFFFFFFu, m);
-        if ((threadIdx.x & 31) == 0) atomicMax(&s_max[i], m);
+        t = __reduce_add_sync(0xFFFFFFFFu, t);
+        if ((threadIdx.x & 31) == 0) {
+            atomicMax(&s.most[i], m);
+            atomicAdd(&s.sum[i], t);
+        }
     }
     __syncthreads();
-    constexpr uint64_t all = kSampleBlocks * 256 * kSamplePerThread;
+    constexpr uint64_t all = kSampleBlocks * 256 * kSamplePerThread; // 2^15 samples of at most 2^6 gates each
     const uint64_t n_cand = ctl->n_cand;
+    auto scaled = [&](uint32_t load) { return n_cand > all ? load * n_cand / all : load; }; // the product is below 2^53
     int best = kLengths - 1;
     uint64_t t_best = 0;
     for (int i = kLengths - 1; i >= 0; --i) {
-        const uint64_t load = n_cand > all ? s_max[i] * n_cand / all : s_max[i]; // below 2^53 (2^21 sampled pairs at most)
-        const uint64_t t = 2500000 + (50000 * load + 150000000 + 20 * n) / window_length(i, most);
+        const uint64_t t = 2500000 + (50000 * scaled(s.most[i]) + 150000000 + 20 * n) / window_length(i, most);
         if (i == kLengths - 1 || t < t_best) {
             best = i;
             t_best = t;
         }
     }
-    return best;
+    const uint64_t len = window_length(best, most), active = scaled(s.sum[best]) / len;
+    t_best -= 50000 * min(scaled(s.most[best]) / len, uint64_t(32));
+    const uint64_t by_gate = 6200000 + 4000 * min(active, uint64_t(1000)) + 65 * active + 3 * n / 2;
+    const uint64_t change = 200000000 / window_length(kLengths - 1, most);
+    return 20 * t_best <= 23 * by_gate + 20 * change ? best : -1;
 }
 
 // Mask and sector of every candidate; one that passes no lower_atol gate of a gate of the window it
@@ -452,13 +474,14 @@ __global__ void __launch_bounds__(256) k_window_count(Store st, WindowScratch ws
     __shared__ uint32_t s_inv[64 * W];
     __shared__ uint32_t s_entries[kMaxSectors];
     __shared__ float s_sin[kWindow];
-    __shared__ uint32_t s_max[kLengths];
+    __shared__ LengthShared s_len;
     WindowCtl *ctl = ws.ctl;
     const uint32_t lo = cnt->step;
     if (cnt->stall != kNoStall || lo >= hi) return;
     const uint32_t n = ctl->n_cand;
     if (n <= blockIdx.x * blockDim.x || window_dense(n, cnt->n)) return;
-    const int len = choose_length(ctl, sectors, hi - lo, cnt->n, s_max);
+    const int len = choose_length(ctl, sectors, hi - lo, cnt->n, s_len);
+    if (len < 0) return;
     const uint64_t in = first_gates(window_length(len, hi - lo));
     for (uint32_t c = threadIdx.x; c < 64 * W; c += blockDim.x) {
         s_mask[c] = ctl->tables.mask[c];
@@ -524,21 +547,21 @@ __global__ void __launch_bounds__(256) k_window_scatter(Store st, WindowScratch 
                                                          const uint64_t *__restrict__ c_mask,
                                                          const uint16_t *__restrict__ c_sector,
                                                          const Counters *__restrict__ cnt, uint32_t hi, uint32_t sectors) {
-    __shared__ uint32_t s_base[kMaxSectors + 1], s_at[kMaxSectors], s_part[8], s_max[kLengths];
+    __shared__ uint32_t s_base[kMaxSectors + 1], s_at[kMaxSectors], s_part[8];
+    __shared__ LengthShared s_len;
     WindowCtl *ctl = ws.ctl;
     const uint32_t lo = cnt->step;
     const bool run = cnt->stall == kNoStall && lo < hi;
     const uint32_t n = ctl->n_cand;
-    const bool dense = run && window_dense(n, cnt->n);
-    if (!run || dense) {
+    if (run && n == 0 && blockIdx.x != 0) return;
+    const int len = run && !window_dense(n, cnt->n) ? choose_length(ctl, sectors, hi - lo, cnt->n, s_len) : -1;
+    if (len < 0) {
         if (blockIdx.x == 0 && threadIdx.x == 0) {
             ctl->run = 0;
-            ctl->overflow = dense ? 3 : 0;
+            ctl->overflow = run ? 3 : 0;
         }
         return;
     }
-    if (n == 0 && blockIdx.x != 0) return;
-    const int len = choose_length(ctl, sectors, hi - lo, cnt->n, s_max);
     const uint32_t K = window_length(len, hi - lo);
     sector_bases(ctl->sector, sectors, s_base, s_part);
     if (blockIdx.x == 0) {
@@ -549,6 +572,7 @@ __global__ void __launch_bounds__(256) k_window_scatter(Store st, WindowScratch 
             ctl->overflow = 0;
             ctl->n_start = cnt->n;
             ctl->n_chunks = s_base[sectors];
+            ctl->grow = max(kGrowChunks, 8 * (n / sectors) / kChunk);
         }
         if (threadIdx.x < kWindow) {
             ctl->anti[threadIdx.x] = 0;
@@ -615,7 +639,7 @@ struct GateShared {
     uint64_t comm[kWindow];
     uint32_t chunk[kSectorChunks]; // the sector's chunks, in list order
     uint32_t anti[kWindow], emitted[kWindow], appended[kWindow];
-    uint32_t n_list[2], n_pass, n_queue, n_join, n_insert, first;
+    uint32_t n_list[2], n_pass, n_queue, n_join, n_insert, first, most_chunks;
     int failed;
 };
 struct GateLists { // sized by the block's T threads
@@ -718,6 +742,7 @@ __global__ void __launch_bounds__(kSectorThreads, kSectorsPerSM)
         if (tid == 0) ctl->overflow = 2;
         return;
     }
+    if (tid == 0) sh.most_chunks = min(kSectorChunks, max(ctl->grow, 4 * n_chunks)); // read by the same thread
     for (uint32_t k = tid; k < n_chunks; k += T) sh.chunk[k] = first + k;
     __syncthreads();
     auto slot_at = [&](uint32_t p) { return sh.chunk[p / kChunk] * kChunk + p % kChunk; };
@@ -763,9 +788,9 @@ __global__ void __launch_bounds__(kSectorThreads, kSectorsPerSM)
                 const uint32_t need = (room + kChunk - 1) / kChunk;
                 if (tid == 0) {
                     for (uint32_t k = n_chunks; k < need; ++k) {
-                        const uint32_t c = k < kSectorChunks ? atomicAdd(&ctl->n_chunks, 1u) : 0u;
-                        if (k >= kSectorChunks || c >= ws.slots / kChunk) {
-                            sh.failed = k >= kSectorChunks ? 2 : 1;
+                        const uint32_t c = k < sh.most_chunks ? atomicAdd(&ctl->n_chunks, 1u) : 0u;
+                        if (k >= sh.most_chunks || c >= ws.slots / kChunk) {
+                            sh.failed = k >= sh.most_chunks ? 2 : 1;
                             break;
                         }
                         sh.chunk[k] = c;

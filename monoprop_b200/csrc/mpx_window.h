@@ -10,6 +10,11 @@ namespace mpx {
 constexpr int kWindow = 64;             // gates per window at most (the masks are 64-bit words)
 constexpr uint32_t kChunk = 1024;       // list slots per chunk of a sector's list
 constexpr uint32_t kSectorChunks = 512; // chunks per sector at most
+// A sector's list may grow to this many chunks, eight times the mean sector's at the window's start or four times its
+// own then, whichever is most; a window in which one grows past that is given up and its gates run one by one. One
+// block has all the terms of a coset, at some 0.05 us each per gate: without a limit a few terms that grow to 1e6 within
+// the window (150 gates on 10 of 161 modes) kept it for 180 ms, 9 ms gate by gate; 4096 terms take 1 ms at most.
+constexpr uint32_t kGrowChunks = 4;
 constexpr uint32_t kMaxSectors = 2048;
 // A window runs only while at most half of the store's terms are candidates (a quarter above kLargeTerms terms).
 // With more, leaving the others aside gains less than the lists cost, and both paths are bound by the emitted
@@ -20,6 +25,9 @@ constexpr uint32_t kMaxSectors = 2048;
 // density (5x3 Hubbard lattice, 6e4 terms: 4.5 ms against 6.2 ms).
 constexpr uint64_t kDenseTerms = uint64_t(1) << 16, kLargeTerms = uint64_t(1) << 22;
 constexpr uint64_t kDenseGates = 192;   // steps taken gate by gate before the next try
+// Fewer steps than this run gate by gate without a try: over 32 gates windows take 1.2 to 1.4 times as long, a try that
+// is declined some 0.1 ms (8 gates: 0.09 ms gate by gate, 0.19 with a try), over 64 gates 0.8 times.
+constexpr uint64_t kLeastGates = 32;
 constexpr int kLengths = 4;             // window lengths tried: kWindow / 8, / 4, / 2 and kWindow gates
 constexpr int kSectorThreads = 128;     // threads of a sector's block
 constexpr int kSectorsPerSM = 8;        // resident blocks per SM it is compiled for; one wave of sectors
@@ -45,10 +53,10 @@ struct WindowCtl {
     uint32_t lo;       // first step of the last window
     uint32_t gates;    // its number of gates
     uint32_t run;      // 1: the window runs (0: an earlier window stalled, its kernels do nothing)
-    uint32_t overflow; // 1: the appends did not fit, 2: a sector's list was full (nothing is committed then),
-                       // 3: too many active terms, the window does not run
+    uint32_t overflow; // 1: the appends did not fit, 2: a sector's list was full or grew too long (nothing is committed then),
+                       // 3: too many active terms or too dear, the window does not run
     uint32_t pending;  // 1: its passive terms still lack their cos factors, its counters their place
-    uint32_t pad;
+    uint32_t grow;     // chunks a sector's list may grow to (kGrowChunks)
     uint64_t n_start;  // store size at its start
     uint64_t comm[kWindow];   // bit j of entry b: gates b and j of the window anticommute
     WindowTables tables;

@@ -1,6 +1,6 @@
-"""When a frozen structure replays in windows (csrc/mpx_replay.cuh) and when gate by gate.
+"""When gates and frozen structures run in windows (csrc/mpx_window.cuh, mpx_replay.cuh) and when gate by gate.
 
-Both replays give the same numbers (test_gpu_replay.py); these tests look at what a call costs, in launches or, where a
+Both give the same numbers (test_gpu_window.py, test_gpu_replay.py); these tests look at what a call costs, in launches or, where a
 wrong choice costs a factor of a hundred, in time.
 """
 
@@ -67,3 +67,21 @@ def test_generators_on_few_modes_do_not_put_the_store_on_one_block(modes):
     circ.close()
     eng.close()
     assert windows <= 5 * gate_by_gate
+
+
+def test_propagation_on_few_modes_does_not_stay_on_one_block():
+    """only_rotate_len_k = all slots changes nothing but the path: gate by gate. Windows in which one block takes the
+    whole store, as it grows from one term to 1e6 in one coset, take some twenty times as long."""
+    wl = on_few_modes(161, 10, 150, 3)
+    seconds, sizes = [], []
+    for k in (None, 2 * wl.num_modes):
+        for _ in range(2):
+            eng = _native.engine_for(wl)
+            eng.set_only_rotate_len_k(k)
+            t = time.perf_counter()
+            eng.propagate(wl.gen_words(), wl.angles())
+            seconds.append(time.perf_counter() - t)
+            sizes.append((eng.size(), eng.expectation()))
+            eng.close()
+    assert sizes[1][0] == sizes[3][0] and abs(sizes[1][1] - sizes[3][1]) <= 1e-12
+    assert seconds[1] <= 5 * seconds[3]
