@@ -1474,13 +1474,13 @@ int generator_rank(const uint64_t *words, uint64_t n, int W) {
 
 // Gates per replay window. A window leaves 2^(rank of the circuit's generators - rank of its own) cosets of every
 // class of terms that the circuit connects, and sectors stay balanced while those are many; longer windows make
-// fewer dense passes. (On the 5x10 lattice, rank 99, 64 gates leave a few hundred occupied cosets, busiest block 8 times the mean,
-// 32 leave it at 1.2-1.4.) Measured per 16 of the rank: 4, 5 and 6 gates give 17.9, 16.8 and 17.2 ms for the reverse
-// sweep of the 50-qubit gradient (8 layers) and 3.23, 2.87 and 2.82 ms per call of the 6x6 Hubbard loop. The rank and
-// not the number of modes: 150 gates on 10 of 161 modes are one coset per 64 gates, and one block replayed 1e6
-// terms (744 ms per gradient, 5.4 ms gate by gate).
+// fewer dense passes. Measured per 16 of the rank: 5, 6, 7 and 8 gates give 2.92, 3.15, 3.10 and 2.66 ms per graph
+// gradient of the 6x6 Hubbard circuit (4 steps), 1.72, 1.61, 1.55 and 1.47 of the 5x5 one, 9.1, 8.8, 8.45 and 8.55 of the
+// 5x10 lattice, 26.7, 26.0, 25.9 and 25.9 of the 10x10 one; logged gradients alike. (Rank 99 on the 5x10 lattice: 32
+// gates leave the busiest block at 1.2-1.4 times the mean, 64 at 8 times.) The rank and not the number of modes: 150 gates on 10
+// of 161 modes are one coset per 64 gates, and one block replayed 1e6 terms (744 ms per gradient, 5.4 ms gate by gate).
 uint32_t replay_window(const CircuitDev &cd) {
-    return static_cast<uint32_t>(std::min<int>(kWindow, std::max(8, (5 * cd.rank + 15) / 16)));
+    return static_cast<uint32_t>(std::min<int>(kWindow, std::max(8, (cd.rank + 1) / 2)));
 }
 
 // Whether a gradient over a frozen structure takes less time in windows than gate by gate. Windows: 64 us for each
