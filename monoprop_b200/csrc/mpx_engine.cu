@@ -1190,6 +1190,7 @@ mpx_status run_range(mpx_engine *eng, const CircuitDev &cd, uint64_t lo, uint64_
     uint64_t chunk_id = 0;
     bool pending = false;
     uint64_t pending_slot = 0;
+    uint64_t rec_seen = 0; // records of a recording pass at the last report
     // Small store: run gates in one shared-memory block until the store outgrows it (or the range ends).
 
     if (e->small_path && e->W <= 4 && !e->profile && !cd.any_cos_zero && !e->tr.has_len_k &&
@@ -1319,9 +1320,14 @@ mpx_status run_range(mpx_engine *eng, const CircuitDev &cd, uint64_t lo, uint64_
                 ++chunk_id;
                 continue;
             }
-            if (e->fwd_tape.r_src != nullptr && e->fwd_tape.r_vs == nullptr && step < hi &&
-                snap.rec_total > e->fwd_tape.r_cap / 4 && snap.rec_total <= e->fwd_tape.r_cap) {
-                // the pair log fills up: more room before the chunks after the one in flight (which may overflow it)
+            // The pair log fills up: more room before the chunks after the one in flight (which may overflow it). A log
+            // of unknown size as soon as a quarter is used; one sized by an earlier pass (rec_hint, and a quarter more)
+            // only when this pass has needed more than that one and what is left might not take the next chunks.
+            const uint64_t used = snap.rec_total, chunk_used = used - std::min<uint64_t>(used, rec_seen);
+            rec_seen = used;
+            const bool filling = e->rec_hint == 0 ? used > e->fwd_tape.r_cap / 4
+                                                  : used > e->rec_hint && used + 4 * chunk_used > e->fwd_tape.r_cap;
+            if (e->fwd_tape.r_src != nullptr && e->fwd_tape.r_vs == nullptr && step < hi && filling && used <= e->fwd_tape.r_cap) {
                 MPX_CUDA(cudaMemcpyAsync(e->h_cnt, e->d_cnt, sizeof(Counters), cudaMemcpyDeviceToHost, e->stream));
                 MPX_CUDA(cudaStreamSynchronize(e->stream));
                 if (e->h_cnt->rec_total <= e->fwd_tape.r_cap) grow_pair_log(e, e->h_cnt->rec_total);
