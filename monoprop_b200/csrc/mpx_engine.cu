@@ -1736,10 +1736,11 @@ mpx_status build_plan(mpx_engine *eng, const CircuitDev &cd, const FrozenGraph &
     if (ce == cudaSuccess) ce = cudaStreamSynchronize(e->stream);
     for (const uint32_t b : busiest) work.busiest += b;
     const bool pays = replay_pays(work, most);
-    for (uint32_t w = 0; ce == cudaSuccess && pays && w < n_win; ++w)
+    if (ce == cudaSuccess && pays && in_vs == nullptr) ce = replay_place(a, q, so, g.src, g.tgt, g.code, g.p_begin, g.p_count);
+    for (uint32_t w = 0; ce == cudaSuccess && pays && in_vs != nullptr && w < n_win; ++w)
         ce = replay_scatter(a, q, so, w, g.src, g.tgt, g.code, in_vs, in_vt, vs, vt, g.p_begin, g.p_count, begin[w * K],
                             range[w]);
-    e->launches += 2 + (pays ? 2 : 1) * n_win;
+    e->launches += 2 + n_win + (!pays ? 0 : in_vs == nullptr ? 1 : n_win);
     for (void *ptr : {static_cast<void *>(so.tables), static_cast<void *>(so.cursor), static_cast<void *>(so.base),
                       static_cast<void *>(so.busiest), static_cast<void *>(so.c_mask),
                       static_cast<void *>(so.c_sector)})
@@ -1803,8 +1804,9 @@ mpx_status replay_gradient(mpx_engine *eng, const CircuitDev &cd, const FrozenGr
     const uint64_t L = g.L, nf = g.n_final;
     uint64_t pairs = 0;
     for (const uint64_t c : g.count) pairs += c;
-    double *vs = nullptr, *vt = nullptr, *lam = nullptr, *grad = nullptr;
+    double *vs = nullptr, *vt = nullptr, *lam = nullptr, *grad = nullptr, *part = nullptr;
     uint8_t *mark = nullptr; // forward: gates applied per term; backward: its earliest pair
+    const ReplayLaunch a = replay_launch(e, cd, g);
     std::vector<double *> ck(p.windows, nullptr);
     cudaError_t ce = cudaSuccess;
     auto A = [&](auto **ptr, uint64_t n) {
@@ -1815,11 +1817,12 @@ mpx_status replay_gradient(mpx_engine *eng, const CircuitDev &cd, const FrozenGr
     A(&vt, pairs);
     A(&lam, nf);
     A(&grad, L);
+    A(&part, static_cast<uint64_t>(kSumWindows) * kWindow * replay_slots(a, p));
     A(&mark, nf);
     for (uint32_t w = 0; w < p.windows; ++w) A(&ck[w], g.n0[static_cast<uint64_t>(w) * p.gates]);
     auto release = [&]() {
         for (void *q : {static_cast<void *>(vs), static_cast<void *>(vt), static_cast<void *>(lam), static_cast<void *>(grad),
-                        static_cast<void *>(mark)})
+                        static_cast<void *>(part), static_cast<void *>(mark)})
             dev_free(e, q);
         for (double *q : ck) dev_free(e, q);
     };
@@ -1828,10 +1831,8 @@ mpx_status replay_gradient(mpx_engine *eng, const CircuitDev &cd, const FrozenGr
         release();
         return MPX_OK;
     }
-    const ReplayLaunch a = replay_launch(e, cd, g);
     const uint64_t n_first = g.n0[0];
     ce = cudaMemsetAsync(mark, 0, std::max<uint64_t>(nf, 4), e->stream);
-    if (ce == cudaSuccess) ce = cudaMemsetAsync(grad, 0, L * sizeof(double), e->stream);
     if (ce == cudaSuccess && n_first > 0)
         ce = cudaMemcpyAsync(ck[0], e->st.coef, n_first * sizeof(double), cudaMemcpyDeviceToDevice, e->stream);
     auto end_of = [&](uint32_t w) { return w + 1 < p.windows ? g.n0[static_cast<uint64_t>(w + 1) * p.gates] : nf; };
@@ -1839,8 +1840,8 @@ mpx_status replay_gradient(mpx_engine *eng, const CircuitDev &cd, const FrozenGr
         ce = replay_forward(a, p, w, end_of(w), mark, vs, vt, w + 1 < p.windows ? ck[w + 1] : nullptr);
     mpx_status s = ce == cudaSuccess ? final_adjoint(e, lam, nf) : MPX_OK;
     for (uint32_t w = p.windows; ce == cudaSuccess && s == MPX_OK && w-- > 0;)
-        ce = replay_reverse(a, p, w, g.n0[static_cast<uint64_t>(w) * p.gates], lam, mark, vs, vt, ck[w], grad);
-    e->launches += 4 * p.windows + 1;
+        ce = replay_reverse(a, p, w, g.n0[static_cast<uint64_t>(w) * p.gates], lam, mark, vs, vt, ck[w], part, grad);
+    e->launches += 4 * p.windows + 1 + (p.windows + kSumWindows - 1) / kSumWindows;
     if (ce == cudaSuccess && s == MPX_OK)
         ce = cudaMemcpyAsync(grad_angles, grad, L * sizeof(double), cudaMemcpyDeviceToHost, e->stream);
     if (ce == cudaSuccess) ce = cudaStreamSynchronize(e->stream);
@@ -1860,7 +1861,7 @@ mpx_status adjoint_backward_logged(mpx_engine *eng, const CircuitDev &cd, const 
     AdjointState &A = e->adj;
     *done = false;
     const uint64_t L = A.L, nf = A.n_final;
-    double *vs = nullptr, *vt = nullptr, *lam = nullptr, *grad = nullptr;
+    double *vs = nullptr, *vt = nullptr, *lam = nullptr, *grad = nullptr, *part = nullptr;
     uint8_t *mark = nullptr;
     ReplayPlan p{};
     cudaError_t ce = cudaSuccess;
@@ -1875,7 +1876,7 @@ mpx_status adjoint_backward_logged(mpx_engine *eng, const CircuitDev &cd, const 
     alloc(&mark, nf);
     auto release = [&]() {
         for (void *q : {static_cast<void *>(vs), static_cast<void *>(vt), static_cast<void *>(lam), static_cast<void *>(grad),
-                        static_cast<void *>(mark)})
+                        static_cast<void *>(part), static_cast<void *>(mark)})
             dev_free(e, q);
         free_plan(e, p);
     };
@@ -1891,13 +1892,18 @@ mpx_status adjoint_backward_logged(mpx_engine *eng, const CircuitDev &cd, const 
         release();
         return s;
     }
-    ce = cudaMemsetAsync(mark, 0, std::max<uint64_t>(nf, 4), e->stream);
-    if (ce == cudaSuccess) ce = cudaMemsetAsync(grad, 0, L * sizeof(double), e->stream);
-    if (ce == cudaSuccess) s = final_adjoint(e, lam, nf);
     const ReplayLaunch a = replay_launch(e, cd, g);
+    alloc(&part, static_cast<uint64_t>(kSumWindows) * kWindow * replay_slots(a, p));
+    if (ce != cudaSuccess) {
+        cudaGetLastError();
+        release();
+        return MPX_OK;
+    }
+    ce = cudaMemsetAsync(mark, 0, std::max<uint64_t>(nf, 4), e->stream);
+    if (ce == cudaSuccess) s = final_adjoint(e, lam, nf);
     for (uint32_t w = p.windows; ce == cudaSuccess && s == MPX_OK && w-- > 0;)
-        ce = replay_reverse(a, p, w, A.ck_n[w], lam, mark, vs, vt, A.ck_coef[w], grad);
-    e->launches += 2 * p.windows + 1;
+        ce = replay_reverse(a, p, w, A.ck_n[w], lam, mark, vs, vt, A.ck_coef[w], part, grad);
+    e->launches += 2 * p.windows + 1 + (p.windows + kSumWindows - 1) / kSumWindows;
     if (ce == cudaSuccess && s == MPX_OK)
         ce = cudaMemcpyAsync(grad_angles, grad, L * sizeof(double), cudaMemcpyDeviceToHost, e->stream);
     if (ce == cudaSuccess) ce = cudaStreamSynchronize(e->stream);

@@ -111,6 +111,7 @@ __global__ void __launch_bounds__(1024) k_replay_prefix(ReplayPlan p, ReplaySort
     if (threadIdx.x == 0) so.busiest[blockIdx.x] = s_most;
 }
 
+// Places the pairs and their logged values, in any order within a sector and gate: the log of a propagation has none of its own.
 __global__ void __launch_bounds__(256) k_replay_scatter(ReplayPlan p, ReplaySort so, uint32_t window, uint32_t L,
                                                          const uint32_t *__restrict__ src, const uint32_t *__restrict__ tgt,
                                                          const int8_t *__restrict__ code, const double *__restrict__ in_vs,
@@ -136,9 +137,44 @@ __global__ void __launch_bounds__(256) k_replay_scatter(ReplayPlan p, ReplaySort
         p.tgt[at] = tgt[r];
         p.code[at] = code[r];
         p.mask[at] = so.c_mask[r];
-        if (in_vs != nullptr) {
-            vs[at] = in_vs[r];
-            vt[at] = in_vt[r];
+        vs[at] = in_vs[r];
+        vt[at] = in_vt[r];
+    }
+}
+
+// The same in the log's order, one block per gate: a structure that is replayed again and again keeps one order of its
+// pairs, whichever engine sorts it (a clone has the same log). Warps take their turns at the sectors' cursors, 32 pairs
+// a turn; a gate of 3e5 pairs takes about half a millisecond, once per structure.
+__global__ void __launch_bounds__(256) k_replay_place(ReplayPlan p, ReplaySort so, const uint32_t *__restrict__ src,
+                                                       const uint32_t *__restrict__ tgt, const int8_t *__restrict__ code,
+                                                       const uint64_t *__restrict__ p_begin,
+                                                       const unsigned long long *__restrict__ p_count) {
+    __shared__ uint32_t s_cursor[kMaxSectors];
+    const uint32_t window = blockIdx.x / p.gates, g = blockIdx.x % p.gates;
+    const uint64_t first = p_begin[blockIdx.x], count = p_count[blockIdx.x];
+    if (count == 0) return;
+    const uint32_t *cursor = so.cursor + static_cast<uint64_t>(window) * p.sectors * p.gates;
+    for (uint32_t s = threadIdx.x; s < p.sectors; s += blockDim.x) s_cursor[s] = cursor[s * p.gates + g];
+    __syncthreads();
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (uint64_t k0 = 0; k0 < count; k0 += blockDim.x) {
+        const uint64_t r = first + k0 + threadIdx.x;
+        const bool in = k0 + threadIdx.x < count;
+        const uint32_t s = in ? so.c_sector[r] : kNoSector;
+        const uint32_t peers = __match_any_sync(0xFFFFFFFFu, s);
+        const uint32_t rank = __popc(peers & ((1u << lane) - 1u));
+        uint32_t at = 0;
+        for (uint32_t w = 0; w < blockDim.x / 32; ++w) {
+            if (w == warp && in) at = s_cursor[s] + rank;
+            __syncwarp();
+            if (w == warp && in && rank == 0) s_cursor[s] = at + __popc(peers);
+            __syncthreads();
+        }
+        if (in) {
+            p.src[at] = src[r];
+            p.tgt[at] = tgt[r];
+            p.code[at] = code[r];
+            p.mask[at] = so.c_mask[r];
         }
     }
 }
@@ -342,10 +378,11 @@ __device__ __forceinline__ void gather_kappa(uint32_t a0, uint32_t a1, double ka
     __syncwarp();
 }
 
-// grad of the window's gates: lane j's acc (times -2 tan) and direct parts of all warps of the block.
-__device__ __forceinline__ void add_gradient(double (*s_sum)[kWindow], double acc0, double acc1, double d0, double d1,
-                                             const GateDesc *__restrict__ gates, uint32_t L, uint32_t lo, uint32_t n,
-                                             double *__restrict__ grad) {
+// The block's share of the derivatives of the window's gates, to its slot of every gate's row: lane j's acc (times
+// -2 tan) and direct parts of all warps, in order.
+__device__ __forceinline__ void block_gradient(double (*s_sum)[kWindow], double acc0, double acc1, double d0, double d1,
+                                               const GateDesc *__restrict__ gates, uint32_t L, uint32_t lo, uint32_t n,
+                                               double *__restrict__ part, uint32_t slots, uint32_t slot) {
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
@@ -359,8 +396,25 @@ __device__ __forceinline__ void add_gradient(double (*s_sum)[kWindow], double ac
     for (uint32_t g = threadIdx.x; g < n; g += blockDim.x) {
         double t = 0.0;
         for (uint32_t w = 0; w < blockDim.x / 32; ++w) t += s_sum[w][g];
-        if (t != 0.0) atomicAdd(&grad[L - 1 - (lo + g)], t);
+        part[static_cast<uint64_t>(g) * slots + slot] = t;
     }
+}
+
+// dE/dangle of the gates of blockIdx.y's window, one block per gate: the sum of its row's slots in a fixed order, so
+// that the bits do not depend on which block came first. 14 values per thread, from L2; a launch for kSumWindows windows.
+__global__ void __launch_bounds__(128) k_reverse_sum(ReplayPlan p, uint32_t window, uint32_t L, const double *__restrict__ part,
+                                                      uint32_t slots, double *__restrict__ grad) {
+    const uint32_t lo = (window + blockIdx.y) * p.gates, g = blockIdx.x;
+    if (lo + g >= L) return;
+    const double *row = part + (static_cast<uint64_t>(blockIdx.y) * kWindow + g) * slots;
+    double t = 0.0;
+    for (uint32_t k = threadIdx.x; k < slots; k += blockDim.x) t += row[k];
+    __shared__ double s_part[4];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xFFFFFFFFu, t, o);
+    if ((threadIdx.x & 31) == 0) s_part[threadIdx.x >> 5] = t;
+    __syncthreads();
+    if (threadIdx.x == 0) grad[L - 1 - (lo + g)] = (s_part[0] + s_part[1]) + (s_part[2] + s_part[3]);
 }
 
 // The reverse sweep over one window's pairs, last gate first. event[i]: 0, or 1 + the earliest gate of the
@@ -368,7 +422,7 @@ __device__ __forceinline__ void add_gradient(double (*s_sum)[kWindow], double ac
 __global__ void __launch_bounds__(kSectorThreads, kSectorsPerSM)
     k_reverse_pairs(double *__restrict__ lam, uint8_t *__restrict__ event, const uint32_t *__restrict__ longb, ReplayPlan p, uint32_t window,
                     const GateDesc *__restrict__ gates, uint32_t L, const double *__restrict__ vs_log,
-                    const double *__restrict__ vt_log, double *__restrict__ grad) {
+                    const double *__restrict__ vt_log, double *__restrict__ part, uint32_t slots) {
     __shared__ double s_cos[kWindow], s_sin[kWindow];
     __shared__ uint64_t s_comm[kWindow];
     __shared__ uint32_t s_seg[kWindow + 1];
@@ -376,7 +430,10 @@ __global__ void __launch_bounds__(kSectorThreads, kSectorsPerSM)
     const uint32_t lo = window * p.gates, n = min(p.gates, L - lo), tid = threadIdx.x, T = blockDim.x;
     const uint32_t lane = tid & 31;
     const uint32_t *seg = p.seg + static_cast<uint64_t>(window) * (p.sectors * p.gates + 1) + blockIdx.x * p.gates;
-    if (seg[0] == seg[p.gates]) return;
+    if (seg[0] == seg[p.gates]) {
+        for (uint32_t g = tid; g < n; g += T) part[static_cast<uint64_t>(g) * slots + blockIdx.x] = 0.0;
+        return;
+    }
     for (uint32_t g = tid; g <= n; g += T) {
         s_seg[g] = seg[g];
         if (g < n) {
@@ -444,7 +501,7 @@ __global__ void __launch_bounds__(kSectorThreads, kSectorsPerSM)
         }
         __syncthreads();
     }
-    add_gradient(s_sum, acc0, acc1, d0, d1, gates, L, lo, n, grad);
+    block_gradient(s_sum, acc0, acc1, d0, d1, gates, L, lo, n, part, slots, blockIdx.x);
 }
 
 // The rest of a reverse window: every term's gates before its first pair (all of them for an unpaired term), for
@@ -452,7 +509,7 @@ __global__ void __launch_bounds__(kSectorThreads, kSectorsPerSM)
 __global__ void __launch_bounds__(kCloseWarps * 32, 3)
     k_reverse_close(Store st, uint32_t parity_col, const uint32_t *__restrict__ longb, double *__restrict__ lam, uint8_t *__restrict__ event,
                     const double *__restrict__ ck, const GateDesc *__restrict__ gates, uint32_t L, uint32_t lo, uint32_t n,
-                    uint64_t n_terms, double *__restrict__ grad) {
+                    uint64_t n_terms, double *__restrict__ part, uint32_t slots, uint32_t first_slot) {
     __shared__ __align__(16) DenseShared s;
     __shared__ double s_sum[kCloseWarps][kWindow], s_kap[kCloseWarps][32];
     dense_setup(s, st, gates, L, lo, n);
@@ -497,7 +554,7 @@ __global__ void __launch_bounds__(kCloseWarps * 32, 3)
         }
         __syncwarp();
     }
-    add_gradient(s_sum, acc0, acc1, 0.0, 0.0, gates, L, lo, n, grad);
+    block_gradient(s_sum, acc0, acc1, 0.0, 0.0, gates, L, lo, n, part, slots, first_slot + blockIdx.x);
 }
 
 } // namespace mpx

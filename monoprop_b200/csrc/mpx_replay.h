@@ -46,13 +46,19 @@ cudaError_t replay_scatter(const ReplayLaunch &a, const ReplayPlan &p, const Rep
                            const double *in_vt, double *vs, double *vt, const uint64_t *p_begin,
                            const unsigned long long *p_count, uint64_t first, uint64_t count);
 
+cudaError_t replay_place(const ReplayLaunch &a, const ReplayPlan &p, const ReplaySort &s, const uint32_t *src,
+                         const uint32_t *tgt, const int8_t *code, const uint64_t *p_begin, const unsigned long long *p_count);
+
 // One window forward: its pairs (vs, vt: logged when not null), then the dense pass over the n_end terms it
 // leaves; ck: the coefficients after the window, when not null. last: [terms] zero between windows.
 cudaError_t replay_forward(const ReplayLaunch &a, const ReplayPlan &p, uint32_t window, uint64_t n_end, uint8_t *last,
                            double *vs, double *vt, double *ck);
 // One window backward: its pairs, then the dense pass over the n_start terms it began with (ck: their
-// coefficients then). Adds dE/dangle of its gates to grad (zeroed by the caller).
+// coefficients then). Every block's share of dE/dangle goes to its slot of part, [kSumWindows][kWindow][replay_slots]
+// by window mod kSumWindows; the window 0 and every kSumWindows-th also adds the slots up to grad.
+constexpr uint32_t kSumWindows = 8;
+inline uint32_t replay_slots(const ReplayLaunch &a, const ReplayPlan &p) { return p.sectors + a.blocks; }
 cudaError_t replay_reverse(const ReplayLaunch &a, const ReplayPlan &p, uint32_t window, uint64_t n_start, double *lam,
-                           uint8_t *event, const double *vs, const double *vt, const double *ck, double *grad);
+                           uint8_t *event, const double *vs, const double *vt, const double *ck, double *part, double *grad);
 
 }  // namespace mpx

@@ -126,12 +126,21 @@ cudaError_t replay_forward(const ReplayLaunch &a, const ReplayPlan &p, uint32_t 
     return cudaGetLastError();
 }
 
+cudaError_t replay_place(const ReplayLaunch &a, const ReplayPlan &p, const ReplaySort &s, const uint32_t *src,
+                         const uint32_t *tgt, const int8_t *code, const uint64_t *p_begin, const unsigned long long *p_count) {
+    k_replay_place<<<a.L, 256, 0, a.stream>>>(p, s, src, tgt, code, p_begin, p_count);
+    return cudaGetLastError();
+}
+
 cudaError_t replay_reverse(const ReplayLaunch &a, const ReplayPlan &p, uint32_t window, uint64_t n_start, double *lam,
-                           uint8_t *event, const double *vs, const double *vt, const double *ck, double *grad) {
-    const uint32_t lo = window * p.gates, n = std::min(p.gates, a.L - lo);
-    k_reverse_pairs<<<p.sectors, kSectorThreads, 0, a.stream>>>(lam, event, a.longb, p, window, a.desc, a.L, vs, vt, grad);
+                           uint8_t *event, const double *vs, const double *vt, const double *ck, double *part, double *grad) {
+    const uint32_t lo = window * p.gates, n = std::min(p.gates, a.L - lo), slots = replay_slots(a, p), at = window % kSumWindows;
+    double *row = part + static_cast<uint64_t>(at) * kWindow * slots;
+    k_reverse_pairs<<<p.sectors, kSectorThreads, 0, a.stream>>>(lam, event, a.longb, p, window, a.desc, a.L, vs, vt, row, slots);
     k_reverse_close<<<a.blocks, kCloseWarps * 32, 0, a.stream>>>(a.st, 64u * a.W, a.longb, lam, event, ck, a.desc, a.L, lo, n,
-                                                                 n_start, grad);
+                                                                 n_start, row, slots, p.sectors);
+    if (at == 0) // windows come last to first
+        k_reverse_sum<<<dim3(p.gates, std::min(kSumWindows, p.windows - window)), 128, 0, a.stream>>>(p, window, a.L, part, slots, grad);
     return cudaGetLastError();
 }
 
