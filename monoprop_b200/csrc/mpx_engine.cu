@@ -1027,7 +1027,7 @@ mpx_status grow_store(mpx_engine *eng, const Counters &snap) {
         // nothing ran: the caller goes on gate by gate
     }
     else if (snap.reason == kStallSector) {
-        // a window's list was full: the store is as it was before the window, its table is not
+        // a window's lists were full: the store is as it was before the window, its table is not
         MPX_CUDA(cudaMemsetAsync(e->st.table, 0xFF, (e->st.tmask + 1) * sizeof(unsigned long long), e->stream));
         pick_table(e->W)(e, 0, n);
     }

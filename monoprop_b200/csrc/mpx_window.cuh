@@ -790,14 +790,14 @@ __global__ void __launch_bounds__(kSectorThreads, kSectorsPerSM)
                     for (uint32_t k = n_chunks; k < need; ++k) {
                         const uint32_t c = k < sh.most_chunks ? atomicAdd(&ctl->n_chunks, 1u) : 0u;
                         if (k >= sh.most_chunks || c >= ws.slots / kChunk) {
-                            sh.failed = k >= sh.most_chunks ? 2 : 1;
+                            sh.failed = 2; // lists, not the store: its capacity may well do
                             break;
                         }
                         sh.chunk[k] = c;
                     }
                 }
                 __syncthreads();
-                if (sh.failed != 0) { // nothing of this window is committed: the host makes room and runs it again
+                if (sh.failed != 0) { // nothing of this window is committed: its gates run one by one
                     if (tid == 0) ctl->overflow = static_cast<uint32_t>(sh.failed);
                     return;
                 }

@@ -53,7 +53,7 @@ struct WindowCtl {
     uint32_t lo;       // first step of the last window
     uint32_t gates;    // its number of gates
     uint32_t run;      // 1: the window runs (0: an earlier window stalled, its kernels do nothing)
-    uint32_t overflow; // 1: the appends did not fit, 2: a sector's list was full or grew too long (nothing is committed then),
+    uint32_t overflow; // 1: the appends did not fit, 2: a sector's list or all of them together are full (nothing is committed then),
                        // 3: too many active terms or too dear, the window does not run
     uint32_t pending;  // 1: its passive terms still lack their cos factors, its counters their place
     uint32_t grow;     // chunks a sector's list may grow to (kGrowChunks)
