@@ -313,7 +313,8 @@ size_t device_available(mpx_engine *e) {
     return free_b;
 }
 
-cudaError_t dev_alloc(mpx_engine *e, void **ptr, size_t bytes) {
+// A block for the engine; see dev_alloc.
+cudaError_t pool_alloc(mpx_engine *e, void **ptr, size_t bytes) {
     BlockCache &c = block_cache();
     if (bytes < kKeepMin || !e->keep_blocks) {
         const cudaError_t ce = cudaMallocFromPoolAsync(ptr, bytes, e->pool, e->stream);
@@ -346,6 +347,18 @@ cudaError_t dev_alloc(mpx_engine *e, void **ptr, size_t bytes) {
     if (ce == cudaSuccess) {
         std::lock_guard<std::mutex> lock(c.mu);
         c.live[*ptr] = cls;
+    }
+    return ce;
+}
+
+bool give_back_window(mpx_engine *e);
+
+// The window scratch is only a faster way to run the gates: where memory runs out, it goes back for the request.
+cudaError_t dev_alloc(mpx_engine *e, void **ptr, size_t bytes) {
+    cudaError_t ce = pool_alloc(e, ptr, bytes);
+    if (ce == cudaErrorMemoryAllocation && give_back_window(e)) {
+        cudaGetLastError();
+        ce = pool_alloc(e, ptr, bytes);
     }
     return ce;
 }
@@ -737,6 +750,17 @@ void free_window(mpx_engine *e) {
                     static_cast<void *>(w.ctl)})
         dev_free(e, p);
     e->ws = WindowScratch{};
+}
+
+void clear_graphs(mpx_engine *e);
+
+// Whether there was a scratch to free. Captured graphs hold its addresses. (Nothing is allocated between the launches
+// of a range that use it but a larger store, which frees it first.)
+bool give_back_window(mpx_engine *e) {
+    if (e->ws.ctl == nullptr) return false;
+    clear_graphs(e);
+    free_window(e);
+    return true;
 }
 
 uint32_t window_sectors(const mpx_engine *e) { return std::min<uint32_t>(kMaxSectors, static_cast<uint32_t>(e->sms * kSectorsPerSM)); }
