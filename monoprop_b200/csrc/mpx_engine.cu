@@ -99,7 +99,7 @@ struct FrozenGraph {
     // such terms and partners are never scaled.
     bool forward_len_k = false;
     ReplayPlan plan{}; // the pairs in replay order (mpx_replay.cuh), built at the first replay; windows = 0: none
-    bool no_plan = false; // no plan can be had (no room, or pairs the plan does not cover)
+    bool no_plan = false; // gate by gate is as fast, or a plan does not cover the pairs (build_plan)
     Frozen view() const {
         return Frozen{src, tgt, code, p_begin, p_count, pared ? last : nullptr, forward_len_k ? longb : nullptr};
     }
@@ -1792,7 +1792,7 @@ const ReplayPlan *graph_plan(mpx_engine *e, const CircuitDev &cd, FrozenGraph &g
     if (g.plan.windows == 0) {
         bool room = true;
         if (build_plan(e, cd, g, nullptr, nullptr, nullptr, nullptr, g.plan, &room) != MPX_OK || g.plan.windows == 0) {
-            g.no_plan = true;
+            g.no_plan = room; // without room for it now, there may be at the next call
             return nullptr;
         }
     }

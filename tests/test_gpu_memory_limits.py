@@ -10,6 +10,7 @@ import pytest
 from test_gpu_window import circuit
 
 from monoprop_b200 import _native
+from monoprop_b200 import workloads as W
 
 pytestmark = pytest.mark.gpu
 
@@ -45,3 +46,25 @@ def test_window_scratch_is_given_back():
         limited = eng.expectation()
     eng.close()
     assert abs(limited - plain) <= 1e-12
+
+
+def test_a_graph_replays_in_windows_once_there_is_room():
+    """Without memory for the sorted pairs (some 500 MiB) a graph replays gate by gate, two launches a gate; later calls
+    try again."""
+    wl = W.ising50(8)
+    eng = _native.engine_for(wl)
+    circ = eng.upload(wl.gen_words(), wl.angles())
+    eng.graph_build(circ)
+
+    def launches():
+        before = eng.launch_count()
+        return eng.graph_expectation(circ), eng.launch_count() - before
+
+    with only_free(16 * MIB):
+        limited = launches()
+    launches()
+    free = launches()
+    circ.close()
+    eng.close()
+    assert abs(limited[0] - free[0]) <= 1e-12
+    assert limited[1] >= 2 * wl.n_layers > wl.n_layers > free[1]
