@@ -1535,13 +1535,10 @@ bool replay_pays(const ReplayWork &r, double most) {
     return windows <= most * (12.1 * static_cast<double>(r.gates) + 2.1e-5 * r.anti + 8.1e-5 * r.pairs);
 }
 
-// Forward pass for the gradient: resets the store to the initial operator, propagates the circuit
-// segment by segment (segment_gates gates each) and saves the coefficient array at every segment start
-// and at the end. With log_all, and when the previous gradient forward pass of this engine says how many
-// undo records the circuit needs and they fit in free device memory, the pass also logs everything the
-// reverse sweep needs (undo log, both values of every pair), so the backward pass replays nothing.
-mpx_status adjoint_forward(mpx_engine *eng, const CircuitDev &cd, uint64_t segment_gates, bool log_all = false) {
+// One try of adjoint_forward; *logging: it logged (or was about to log) all that the reverse sweep needs.
+mpx_status adjoint_pass(mpx_engine *eng, const CircuitDev &cd, uint64_t segment_gates, bool log_all, bool *logging) {
     mpx_engine *e = eng;
+    *logging = false;
     free_adjoint(e);
     mpx_status s = load_initial(e);
     if (s != MPX_OK) return s;
@@ -1592,6 +1589,7 @@ mpx_status adjoint_forward(mpx_engine *eng, const CircuitDev &cd, uint64_t segme
                 e->fwd_tape.r_vs = A.r_vs;
                 e->fwd_tape.r_vt = A.r_vt;
                 K = replay_window(cd);
+                *logging = true;
             }
             else {
                 cudaGetLastError(); // no room after all: the backward pass replays segments
@@ -1608,10 +1606,7 @@ mpx_status adjoint_forward(mpx_engine *eng, const CircuitDev &cd, uint64_t segme
         e->adj.seg_lo.push_back(lo);
         e->adj.ck_n.push_back(n);
         s = run_range(e, cd, lo, std::min(L, lo + K));
-        if (s != MPX_OK) {
-            free_adjoint(e);
-            return s;
-        }
+        if (s != MPX_OK) return s;
         n = e->h_cnt->n;
     }
     if (e->fwd_tape.r_src != nullptr) {
@@ -1655,6 +1650,23 @@ mpx_status adjoint_forward(mpx_engine *eng, const CircuitDev &cd, uint64_t segme
     e->ck_hint = 0;
     for (uint64_t st = 0; st < L; st += window) e->ck_hint += e->adj.stats[4 * st];
     return MPX_OK;
+}
+
+// Forward pass for the gradient: resets the store to the initial operator, propagates the circuit
+// segment by segment (segment_gates gates each) and saves the coefficient array at every segment start
+// and at the end, and the pairs every gate rotates. With log_all, and when the last pass of this circuit found that it pays (replay_pays) and
+// what it needs fits in free device memory, the segments are replay windows and both values of every pair are
+// logged too, so that the backward pass replays nothing. What fits was estimated from that last pass: other angles may need
+// more checkpoints, and a pass that runs out of memory for them is made again without the log.
+mpx_status adjoint_forward(mpx_engine *e, const CircuitDev &cd, uint64_t segment_gates, bool log_all = false) {
+    bool logging = false;
+    mpx_status s = adjoint_pass(e, cd, segment_gates, log_all, &logging);
+    if (s == MPX_ERR_NOMEM && logging) {
+        e->log_pays = 0;
+        s = adjoint_pass(e, cd, segment_gates, log_all, &logging);
+    }
+    if (s != MPX_OK) free_adjoint(e);
+    return s;
 }
 
 // Values the replay starts terms [lo, hi) of the final store from: the reference-state score in the
