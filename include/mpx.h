@@ -281,7 +281,8 @@ MPX_API mpx_status mpx_update_initial_operator(mpx_engine *e, const uint64_t *wo
  * operator_memory_bytes / operator_memory_breakdown / graph_memory_bytes (binder.h:252-273,
  * MonomialPropagator.h:124-135): keys and coefficients at the store's capacity, the hash table, the
  * bit-column anticommutation index (the reference's InvertedIndex), per-gate scratch, the initial
- * operator, and the frozen graph (pairs and per-step arrays). */
+ * operator, and the frozen graph (pairs, per-step arrays and, from its first windowed replay on, the pairs in replay
+ * order: 17 bytes each and 4 per sector and gate). */
 typedef struct {
     uint64_t terms, capacity;
     uint32_t words;

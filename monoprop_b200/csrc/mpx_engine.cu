@@ -1699,6 +1699,16 @@ void free_plan(mpx_engine *e, ReplayPlan &p) {
     p = ReplayPlan{};
 }
 
+uint64_t plan_bytes(const FrozenGraph &g) {
+    const ReplayPlan &p = g.plan;
+    if (p.windows == 0) return 0;
+    uint64_t pairs = 0;
+    for (const uint64_t c : g.count) pairs += c;
+    return pairs * (2 * sizeof(uint32_t) + sizeof(int8_t) + sizeof(uint64_t)) +
+           static_cast<uint64_t>(p.windows) *
+               ((static_cast<uint64_t>(p.sectors) * p.gates + 1) * sizeof(uint32_t) + kWindow * sizeof(uint64_t));
+}
+
 ReplayLaunch replay_launch(const mpx_engine *e, const CircuitDev &cd, const FrozenGraph &g) {
     return ReplayLaunch{e->st, g.forward_len_k ? g.longb : nullptr, cd.d_desc, static_cast<uint32_t>(cd.n), e->W, static_cast<unsigned>(4 * e->sms), e->stream};
 }
@@ -3334,7 +3344,7 @@ mpx_status mpx_memory(mpx_engine *e, mpx_memory_info *out) {
                                 : pairs * (2 * sizeof(uint32_t) + sizeof(int8_t)) +
                                       g.L * (sizeof(uint64_t) + sizeof(unsigned long long)) +
                                       g.L * static_cast<uint64_t>(e->grid) * kWarps * sizeof(uint32_t) +
-                                      ((g.n_final + 31) / 32) * sizeof(uint32_t);
+                                      ((g.n_final + 31) / 32) * sizeof(uint32_t) + plan_bytes(g);
     return MPX_OK;
 }
 

@@ -1,4 +1,7 @@
-"""The pair log of a recording forward pass (mpx_graph_build, mpx_adjoint_forward) on an engine that has recorded before."""
+"""The pair log of a recording forward pass (mpx_graph_build, mpx_adjoint_forward) on an engine that has recorded before,
+and what a graph is reported to hold."""
+
+import ctypes as C
 
 import pytest
 
@@ -31,3 +34,24 @@ def test_rebuilding_a_graph_holds_no_more_memory():
     circ.close()
     eng.close()
     assert used[1] <= used[0] + (128 << 20) and used[2] <= used[0] + (128 << 20)
+
+
+def test_reported_graph_bytes_count_the_replay_order():
+    """Sorted for windowed replays, a pair takes another 17 bytes: two terms, the phase and the gate mask."""
+    wl = W.ising50(5)
+    eng = _native.engine_for(wl)
+    circ = eng.upload(wl.gen_words(), wl.angles())
+    eng.graph_build(circ)
+
+    def memory():
+        info = _native.MemoryInfo()
+        eng._check(eng.lib.mpx_memory(eng.h, C.byref(info)))
+        return info
+
+    built = memory()
+    eng.graph_expectation(circ)
+    replayed = memory()
+    circ.close()
+    eng.close()
+    assert built.graph_pairs == replayed.graph_pairs > 0
+    assert replayed.graph_bytes >= built.graph_bytes + 17 * built.graph_pairs
