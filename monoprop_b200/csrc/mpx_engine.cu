@@ -1078,6 +1078,30 @@ cudaError_t start_windows(mpx_engine *e, uint64_t at) {
     return ce != cudaSuccess ? ce : cudaMemcpyAsync(&e->d_cnt->step, &from, sizeof(from), cudaMemcpyHostToDevice, e->stream);
 }
 
+// At least n timing events.
+cudaError_t ensure_events(mpx_engine *e, size_t n) {
+    while (e->pev.size() < n) {
+        cudaEvent_t ev = nullptr;
+        const cudaError_t ce = cudaEventCreate(&ev);
+        if (ce != cudaSuccess) return ce;
+        e->pev.push_back(ev);
+    }
+    return cudaSuccess;
+}
+
+// Adds the times between the first two, and the second two, of every four events [4 lo, 4 hi), all completed.
+cudaError_t add_times(mpx_engine *e, size_t lo, size_t hi) {
+    for (size_t k = lo; k < hi; ++k) {
+        float a = 0.f, b = 0.f;
+        cudaError_t ce = cudaEventElapsedTime(&a, e->pev[4 * k], e->pev[4 * k + 1]);
+        if (ce == cudaSuccess) ce = cudaEventElapsedTime(&b, e->pev[4 * k + 1], e->pev[4 * k + 2]);
+        if (ce != cudaSuccess) return ce;
+        e->t_sweep_ms += a;
+        e->t_resolve_ms += b;
+    }
+    return cudaSuccess;
+}
+
 cudaError_t issue_window(mpx_engine *e, const WindowLaunch &w, uint64_t hi, cudaEvent_t *ev) {
     if (ev) cudaEventRecord(ev[0], e->stream);
     cudaError_t ce = window_close(w, static_cast<uint32_t>(hi));
@@ -1122,6 +1146,7 @@ mpx_status run_windows(mpx_engine *eng, const CircuitDev &cd, uint64_t *step, ui
                 known = snap.stall;
                 if (snap.reason != kStallStore || !ensure_window(e)) {
                     *step = known;
+                    MPX_CUDA(add_times(e, 0, timed));
                     return MPX_OK;
                 }
                 MPX_CUDA(start_windows(e, known));
@@ -1140,15 +1165,9 @@ mpx_status run_windows(mpx_engine *eng, const CircuitDev &cd, uint64_t *step, ui
     ++e->launches;
     MPX_CUDA(window_finish(window_launch(e, cd))); // the last window's cos factors and counters
     *step = hi;
-    if (e->profile) {
+    if (timed > 0) {
         MPX_CUDA(cudaStreamSynchronize(e->stream));
-        for (size_t k = 0; k < timed; ++k) {
-            float a = 0.f, b = 0.f;
-            MPX_CUDA(cudaEventElapsedTime(&a, e->pev[4 * k], e->pev[4 * k + 1]));
-            MPX_CUDA(cudaEventElapsedTime(&b, e->pev[4 * k + 1], e->pev[4 * k + 2]));
-            e->t_sweep_ms += a;
-            e->t_resolve_ms += b;
-        }
+        MPX_CUDA(add_times(e, 0, timed));
     }
     return MPX_OK;
 }
@@ -1201,13 +1220,7 @@ mpx_status run_range(mpx_engine *eng, const CircuitDev &cd, uint64_t lo, uint64_
         e->aux_on = true;
         MPX_CUDA(dev_alloc(e, reinterpret_cast<void **>(&e->sc.aux), e->st.cap * sizeof(double)));
     }
-    if (e->profile) {
-        while (e->pev.size() < 4 * L) {
-            cudaEvent_t ev = nullptr;
-            MPX_CUDA(cudaEventCreate(&ev));
-            e->pev.push_back(ev);
-        }
-    }
+    if (e->profile) MPX_CUDA(ensure_events(e, 4 * L));
     const GateFn gate = pick_gate(e->W, e->cfg.basis);
     constexpr uint64_t kChunkGates = 48;
     uint64_t step = lo;
@@ -1299,7 +1312,7 @@ mpx_status run_range(mpx_engine *eng, const CircuitDev &cd, uint64_t lo, uint64_
         uint64_t ran = 0;
         const mpx_status ws = run_windows(e, cd, &step, hi, in_flight, &ran);
         apart = ran > 0 ? kDenseGates : 2 * apart;
-        stretch = e->profile ? hi : std::min(hi, step + apart); // one kind of timing after the other
+        stretch = std::min(hi, step + apart);
         ran_as.push_back({ran, step, stretch});
         return ws;
     };
@@ -1307,13 +1320,15 @@ mpx_status run_range(mpx_engine *eng, const CircuitDev &cd, uint64_t lo, uint64_
         s = run_windows_from(replayed);
         if (s != MPX_OK) return s;
     }
-    const uint64_t by_gate = step; // the first step that runs gate by gate
+    uint64_t by_gate = step; // the first step of the last stretch that runs gate by gate
     for (;;) {
         bool issued = false;
         if (step == stretch && stretch < hi && !pending) {
             if (hi - step >= kLeastGates && ensure_window(e)) {
+                if (e->profile) MPX_CUDA(add_times(e, by_gate, step)); // the windows' events are the same ones
                 s = run_windows_from(false);
                 if (s != MPX_OK) return s;
+                by_gate = step;
             }
             else {
                 stretch = hi;
@@ -1409,13 +1424,7 @@ mpx_status run_range(mpx_engine *eng, const CircuitDev &cd, uint64_t lo, uint64_
         cudaGetLastError();
     }
     if (e->profile) {
-        for (uint64_t st = by_gate; st < hi; ++st) {
-            float a = 0.f, b = 0.f;
-            MPX_CUDA(cudaEventElapsedTime(&a, e->pev[4 * st], e->pev[4 * st + 1]));
-            MPX_CUDA(cudaEventElapsedTime(&b, e->pev[4 * st + 1], e->pev[4 * st + 2]));
-            e->t_sweep_ms += a;
-            e->t_resolve_ms += b;
-        }
+        MPX_CUDA(add_times(e, by_gate, hi));
         e->n_sweep = hi - lo;
     }
     if (e->h_cnt->err != 0)
