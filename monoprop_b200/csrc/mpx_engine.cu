@@ -1127,6 +1127,7 @@ mpx_status run_windows(mpx_engine *eng, const CircuitDev &cd, uint64_t *step, ui
         bool issued = false;
         const uint64_t least = !pending ? 0 : (graph ? hi : window_length(0, kWindow));
         if (known + least < hi) {
+            if (e->profile) MPX_CUDA(ensure_events(e, 4 * (timed + 1))); // a window that is run again has its own
             MPX_CUDA(issue_window(e, window_launch(e, cd), hi, e->profile ? &e->pev[4 * timed] : nullptr));
             timed += e->profile ? 1 : 0;
             MPX_CUDA(cudaMemcpyAsync(&e->h_snap[id & 1], e->d_cnt, sizeof(Counters), cudaMemcpyDeviceToHost, e->stream));

@@ -32,3 +32,19 @@ def test_profiled_propagation_takes_the_same_path():
         eng.close()
     assert abs(launches[1] - launches[0]) <= 0.1 * launches[0]
     assert abs(values[1] - values[0]) <= 1e-12
+
+
+def test_windows_that_are_run_again_are_timed():
+    """A store that starts at its smallest grows several times within the windows of one short circuit."""
+    rng = np.random.default_rng(2)
+    slots = [tuple(sorted(rng.choice(24, size=2, replace=False).tolist())) for _ in range(40)]
+    wl = W.Workload("grow", "pauli", 161, slots, np.ones(40), np.arange(40), rng.uniform(0.3, 1.0, size=40),
+                    {(0, 1): 1.0 + 0j, (4, 5): 0.5 + 0j}, [], 12, "support", 1e-6)
+    out = []
+    for on in (False, True):
+        eng = _native.engine_for(wl, capacity_hint=1)
+        eng.set_profiling(on)
+        eng.propagate(wl.gen_words(), wl.angles())
+        out.append((eng.size(), eng.expectation()))
+        eng.close()
+    assert out[0][0] == out[1][0] and abs(out[0][1] - out[1][1]) <= 1e-12
