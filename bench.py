@@ -429,16 +429,17 @@ def main() -> None:
     h2d = int(gw.nbytes + ang.nbytes + keys.nbytes + coefs.nbytes)
 
     peak, peak_kind = _peaks()
-    # What the path cannot do without, against the whole step: per gate the anticommuting coefficients read and
-    # written and the appended rows written (the store exceeds L2). sweep_bytes is what a gate-by-gate sweep over
-    # the bit-columns moves for the same circuit.
-    floor_bytes = float((16 * anti + (8 * W + 8) * app).sum())
+    # Bytes that gates in windows cannot do without, against the whole step (the store exceeds L2): every gate's
+    # columns once, every coefficient read and written once per 64 gates, the appended rows written. The lists, key
+    # rows and table slots of the active terms come on top, and the gates that run one by one move sweep_bytes' share.
+    floor_bytes = float((fold * n / 8 + 16 * n / 64 + (8 * W + 8) * app).sum())
     achieved = floor_bytes / (ms_per_step * 1e-3) / 1e9
     roofline = {"bound": "hbm", "kernel": "window kernels (whole step)", "achieved": achieved, "peak": peak, "unit": "GB/s",
                 "frac": achieved / peak, "peak_source": f"{peak_kind} hbm_gbs",
                 "traffic": None, "algorithmic_bytes_per_step": floor_bytes, "gate_by_gate_bytes_per_step": sweep_bytes,
-                "kernel_ms_per_step": {"dense passes": statistics.mean(sweep_ms),
-                                       "lists, gates, commit": statistics.mean(resolve_ms)},
+                # of the profiled steps, which take the same path (without programmatic overlap)
+                "kernel_ms_per_step": {"dense passes, sweeps": statistics.mean(sweep_ms),
+                                       "lists, gates, commit, resolves": statistics.mean(resolve_ms)},
                 "path_bytes_per_step": path_bytes,
                 # per step: anticommuting terms (cos-scaled), emitted sine branches, appended partners
                 "anticommuting_per_step": int(anti.sum()), "emitted_per_step": int(emitted.sum()),

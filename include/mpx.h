@@ -172,12 +172,14 @@ MPX_API mpx_status mpx_graph_replay_count(mpx_engine *e, uint64_t *out);
  * coefficient array every segment_gates gates (0 = one segment) and returns <0|O|0>; the engine then holds
  * the evolved operator. mpx_adjoint_backward replays each segment from its checkpoint and returns
  * grad_angles[l] = d<0|O|0>/d(angle_l) for every circuit layer l, angle_l = theta[map_l] * g_l (host
- * buffer of c's n_layers doubles). Peak extra memory: the checkpoints plus, for the largest segment,
- * 12 bytes per anticommuting term-gate pair and 25 bytes per emitted sine branch. Once an engine has run
- * one gradient forward pass it knows how many undo records the circuit needs; when they (12 bytes each,
- * plus 16 bytes per recorded pair) fit in free device memory with room to spare, the next forward pass
- * logs them all and mpx_adjoint_backward runs the reverse sweep alone, without replaying segments
- * (mpx_adjoint_logged reports which). The gradient is the same either way. */
+ * buffer of c's n_layers doubles). Peak extra memory: the checkpoints plus, for the largest segment that is replayed
+ * gate by gate, 12 bytes per anticommuting term-gate pair and 25 bytes per emitted sine branch; a single segment
+ * whose pairs replay in windows takes 33 bytes per pair and a checkpoint per window instead. Once an engine has run
+ * one gradient forward pass of a circuit it knows its pairs and store sizes; where a windowed reverse sweep is
+ * predicted to pay and both values of every pair (16 bytes, twice while they are sorted) and a checkpoint per
+ * window fit in free device memory with room to spare, the next forward pass logs them and
+ * mpx_adjoint_backward runs the reverse sweep alone, without replaying segments (mpx_adjoint_logged reports
+ * which). The gradient is the same either way, up to the order of its sums. */
 MPX_API mpx_status mpx_adjoint_forward(mpx_engine *e, const mpx_circuit *c, uint64_t segment_gates, double *expectation);
 MPX_API mpx_status mpx_adjoint_backward(mpx_engine *e, const mpx_circuit *c, double *grad_angles);
 /* *out = 1 if the last mpx_adjoint_forward logged everything the reverse sweep needs, else 0. */
@@ -237,7 +239,7 @@ MPX_API mpx_status mpx_graph_gradient(mpx_engine *e, const mpx_circuit *c, uint6
  * expectation_value[_and_gradient]_functional: pare_graph, PareGraph.cpp:103-141, keep set
  * indices_above(threshold), MonomialPropagator.inl:950-960). Terms whose reference-state weight exceeds
  * threshold are kept, and walking the layers backward so is every term whose value can still flow into a
- * kept one; later mpx_graph_expectation / mpx_graph_gradient calls skip the cos scaling of every other
+ * kept one; later mpx_graph_expectation / mpx_graph_gradient calls replay gate by gate and skip the cos scaling of every other
  * term and the rotation of pairs with no kept endpoint. <0|O|0> and its gradient are unchanged for
  * threshold in [0, 1) (fully paired terms have weight 1); the replayed coefficients of pared terms are not
  * meaningful. threshold < 0 turns paring off. */
@@ -254,8 +256,10 @@ MPX_API mpx_status mpx_set_pair_log(mpx_engine *e, int64_t capacity);
 /* Per-kernel timing. With profiling on, the launches of every window of gates (the dense pass; the window's
  * lists, gates and commit) or, gate by gate, the sweep and resolve launches are bracketed by CUDA events on the
  * engine stream; mpx_kernel_times returns their summed device time (ms) for the last propagate call: sweep_ms the
- * dense passes and sweeps, resolve_ms the rest. columns_ms is 0: no column launch of its own remains. The reference has no device kernels; this replaces nothing there (its
- * closest counterpart is the per-layer wall time the bench harness records, benches/bench_models.py). */
+ * dense passes and sweeps, resolve_ms the rest. The path is the one that runs unprofiled, but for the shared-memory
+ * block of small stores and the programmatic overlap of launches. columns_ms is 0: no column launch of its own
+ * remains. The reference has no device kernels; this replaces nothing there (its closest counterpart is the
+ * per-layer wall time the bench harness records, benches/bench_models.py). */
 MPX_API mpx_status mpx_set_profiling(mpx_engine *e, int32_t on);
 MPX_API mpx_status mpx_kernel_times(mpx_engine *e, double *sweep_ms, double *resolve_ms, double *columns_ms,
                                     uint64_t *n_gates);

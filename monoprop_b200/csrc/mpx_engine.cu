@@ -1,11 +1,13 @@
 // mpx_engine.cu -- host engine and C ABI (include/mpx.h) of the B200 propagation engine.
 //
-// The engine owns one CUDA stream and a device-resident term store. A propagate call uploads the
-// circuit once as per-gate descriptors, then issues two kernels per gate with no host round trip per
-// gate: the sweep kernel refuses to start a gate that could overflow the store (it records the step and
-// every later launch becomes a no-op), and the host, which checks the counters once per chunk of gates,
-// grows the store and re-issues from that step. Truncation semantics follow the reference's fused
-// ContractImmediately path (MonomialPropagator.inl:594-618).
+// The engine owns one CUDA stream and a device-resident term store. A propagate call uploads the circuit once as
+// per-gate descriptors. A small store runs its gates in one shared-memory block (mpx_small.cuh); a larger one in
+// windows of up to 64 gates (mpx_window.cuh) or, where windows are declined or do not apply, with two kernels per gate
+// (mpx_kernels.cuh). There is no host round trip per gate: a window whose appends do not fit changes nothing, and the
+// sweep kernel refuses to start a gate that could overflow the store; either records the step, every later launch
+// becomes a no-op, and the host, which checks the counters once per window or chunk of gates, grows the store and
+// re-issues from that step. Truncation semantics follow the reference's fused ContractImmediately path
+// (MonomialPropagator.inl:594-618).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -765,9 +767,9 @@ bool give_back_window(mpx_engine *e) {
 
 uint32_t window_sectors(const mpx_engine *e) { return std::min<uint32_t>(kMaxSectors, static_cast<uint32_t>(e->sms * kSectorsPerSM)); }
 
-// List slots of the window path for capacity `cap`: above kLargeTerms terms at most a quarter is active when a
-// window starts (twice that leaves room for those that join), and each sector's last chunk may be partly used. (A window that needs more is run again
-// with a grown store.)
+// List slots of the window path for capacity `cap`: above kLargeTerms terms at most a quarter is active when a window
+// starts (twice that leaves room for those that join), and each sector's last chunk may be partly used. (A window that
+// needs more is given up, and its gates run one by one.)
 uint64_t window_slots(const mpx_engine *e, uint64_t cap) {
     const uint64_t terms = std::min(cap, std::max(cap / 2, kLargeTerms));
     return (terms / kChunk + 2 * window_sectors(e) + 2) * kChunk;
@@ -1116,7 +1118,7 @@ cudaError_t issue_window(mpx_engine *e, const WindowLaunch &w, uint64_t hi, cuda
 // windows until one reports the end of the range, one ahead of the last report (unless the window in flight is
 // sure to end it). in_flight: a captured graph of windows has been launched and reports to h_snap[0]. *ran: how
 // many windows applied gates. Returns with *step < hi when windows cannot go on (no room for their scratch at
-// the grown capacity, or a sector's list over its limit): the caller goes on gate by gate.
+// the grown capacity, full lists, or gates that are cheaper one by one): the caller goes on gate by gate.
 mpx_status run_windows(mpx_engine *eng, const CircuitDev &cd, uint64_t *step, uint64_t hi, bool in_flight, uint64_t *ran) {
     mpx_engine *e = eng;
     bool pending = in_flight, graph = in_flight;
@@ -1513,12 +1515,13 @@ int generator_rank(const uint64_t *words, uint64_t n, int W) {
 }
 
 // Gates per replay window. A window leaves 2^(rank of the circuit's generators - rank of its own) cosets of every
-// class of terms that the circuit connects, and sectors stay balanced while those are many; longer windows make
-// fewer dense passes. Measured per 16 of the rank: 5, 6, 7 and 8 gates give 2.92, 3.15, 3.10 and 2.66 ms per graph
-// gradient of the 6x6 Hubbard circuit (4 steps), 1.72, 1.61, 1.55 and 1.47 of the 5x5 one, 9.1, 8.8, 8.45 and 8.55 of the
-// 5x10 lattice, 26.7, 26.0, 25.9 and 25.9 of the 10x10 one; logged gradients alike. (Rank 99 on the 5x10 lattice: 32
-// gates leave the busiest block at 1.2-1.4 times the mean, 64 at 8 times.) The rank and not the number of modes: 150 gates on 10
-// of 161 modes are one coset per 64 gates, and one block replayed 1e6 terms (744 ms per gradient, 5.4 ms gate by gate).
+// class of terms that the circuit connects, and sectors stay balanced while those are many; longer windows make fewer
+// dense passes. Measured per 16 of the rank: 5, 6, 7 and 8 gates give 2.92, 3.15, 3.10 and 2.66 ms per graph gradient
+// of the 6x6 Hubbard circuit (4 steps), 1.72, 1.61, 1.55 and 1.47 of the 5x5 one, 9.1, 8.8, 8.45 and 8.55 of the 5x10
+// lattice, 26.7, 26.0, 25.9 and 25.9 of the 10x10 one; logged gradients alike. (Rank 99 on the 5x10 lattice: 32 gates
+// leave the busiest block at 1.2-1.4 times the mean, 64 at 8 times.) The rank and not the number of modes: 150 gates
+// on 10 of 161 modes are one coset per 64 gates, and one block replayed 1e6 terms (744 ms per gradient, 5.4 ms gate by
+// gate).
 uint32_t replay_window(const CircuitDev &cd) {
     return static_cast<uint32_t>(std::min<int>(kWindow, std::max(8, (cd.rank + 1) / 2)));
 }
@@ -1662,12 +1665,12 @@ mpx_status adjoint_pass(mpx_engine *eng, const CircuitDev &cd, uint64_t segment_
     return MPX_OK;
 }
 
-// Forward pass for the gradient: resets the store to the initial operator, propagates the circuit
-// segment by segment (segment_gates gates each) and saves the coefficient array at every segment start
-// and at the end, and the pairs every gate rotates. With log_all, and when the last pass of this circuit found that it pays (replay_pays) and
-// what it needs fits in free device memory, the segments are replay windows and both values of every pair are
-// logged too, so that the backward pass replays nothing. What fits was estimated from that last pass: other angles may need
-// more checkpoints, and a pass that runs out of memory for them is made again without the log.
+// Forward pass for the gradient: resets the store to the initial operator, propagates the circuit segment by segment
+// (segment_gates gates each) and saves the coefficient array at every segment start and at the end, and the pairs
+// every gate rotates. With log_all, and when the last pass of this circuit found that it pays (replay_pays) and what
+// it needs fits in free device memory, the segments are replay windows and both values of every pair are logged too,
+// so that the backward pass replays nothing. What fits was estimated from that last pass: other angles may need more
+// checkpoints, and a pass that runs out of memory for them is made again without the log.
 mpx_status adjoint_forward(mpx_engine *e, const CircuitDev &cd, uint64_t segment_gates, bool log_all = false) {
     bool logging = false;
     mpx_status s = adjoint_pass(e, cd, segment_gates, log_all, &logging);
@@ -1908,9 +1911,9 @@ mpx_status replay_gradient(mpx_engine *eng, const CircuitDev &cd, const FrozenGr
     return MPX_OK;
 }
 
-// Reverse sweep over the logs of a forward pass that logged everything (AdjointState::log_ok): the pairs are
-// sorted into replay order with their values, and the windows swept from the checkpoints at their starts. No
-// replay. *done = false (MPX_OK): no room for the sorted pairs, or sectors too unbalanced; the caller replays the segments.
+// Reverse sweep over the logs of a forward pass that logged everything (AdjointState::log_ok): the pairs are sorted
+// into replay order with their values, and the windows swept from the checkpoints at their starts. No replay. *done =
+// false (MPX_OK): no room for the sorted pairs, or sectors too unbalanced; the caller replays the segments.
 mpx_status adjoint_backward_logged(mpx_engine *eng, const CircuitDev &cd, const FrozenGraph &g, double *grad_angles,
                                    bool *done) {
     mpx_engine *e = eng;

@@ -802,8 +802,9 @@ __global__ void __launch_bounds__(kBlock, kSweepBlocksPerSM) k_resolve(Store st,
             }
         }
         // Unique appends (forward) or pair records (replay): one counter bump per round. A recording forward pass
-        // reserves its records (rotated pairs and appends) between the same two barriers, by another thread:
-        // barriers and a second round trip of their own made the 50-qubit gradient's forward pass 31.8 instead of 31.3 ms.
+        // reserves its records (rotated pairs and appends) between the same two barriers, by another thread, which saves
+        // two barriers and a round trip a round. (The 50-qubit gradient's forward pass does not show it: its passes
+        // differ by more than the half millisecond that it once measured.)
         const uint32_t ball = __ballot_sync(0xFFFFFFFFu, REPLAY ? rec : miss);
         const bool recording = !REPLAY && tp.r_src != nullptr;
         const uint32_t rb = recording ? __ballot_sync(0xFFFFFFFFu, rec || miss) : 0u;

@@ -111,7 +111,8 @@ __global__ void __launch_bounds__(1024) k_replay_prefix(ReplayPlan p, ReplaySort
     if (threadIdx.x == 0) so.busiest[blockIdx.x] = s_most;
 }
 
-// Places the pairs and their logged values, in any order within a sector and gate: the log of a propagation has none of its own.
+// Places the pairs and their logged values, in any order within a sector and gate: the log of a propagation has none
+// of its own.
 __global__ void __launch_bounds__(256) k_replay_scatter(ReplayPlan p, ReplaySort so, uint32_t window, uint32_t L,
                                                          const uint32_t *__restrict__ src, const uint32_t *__restrict__ tgt,
                                                          const int8_t *__restrict__ code, const double *__restrict__ in_vs,
@@ -401,7 +402,8 @@ __device__ __forceinline__ void block_gradient(double (*s_sum)[kWindow], double 
 }
 
 // dE/dangle of the gates of blockIdx.y's window, one block per gate: the sum of its row's slots in a fixed order, so
-// that the bits do not depend on which block came first. 14 values per thread, from L2; a launch for kSumWindows windows.
+// that the bits do not depend on which block came first. 14 values per thread, from L2; a launch for kSumWindows
+// windows.
 __global__ void __launch_bounds__(128) k_reverse_sum(ReplayPlan p, uint32_t window, uint32_t L, const double *__restrict__ part,
                                                       uint32_t slots, double *__restrict__ grad) {
     const uint32_t lo = (window + blockIdx.y) * p.gates, g = blockIdx.x;

@@ -13,7 +13,8 @@
 //     terms out to sectors, one thread block each, and a block runs all gates of the window on its sector with
 //     block barriers only: no grid-wide synchronisation, no launch per gate, and no wait for the slowest block
 //     at every gate. Longer windows spread the cost of the dense pass, shorter ones split the store into more
-//     cosets; k_window_sample measures the sectors' loads for four lengths and the window takes the best.
+//     cosets; k_window_sample measures the sectors' loads for four lengths and the window takes the best, or
+//     none where gate by gate takes less time (choose_length).
 // One window is
 //   k_window_close   one dense pass: the previous window's pending cos factors for its passive terms (in gate
 //                    order, so every coefficient is rounded as gate-by-gate scaling rounds it), its counters,
@@ -154,11 +155,11 @@ __device__ __forceinline__ uint32_t more_columns(const GateDesc &gd, const Store
     return a;
 }
 
-// Applies the pending window (ctl) to its passive terms and collects the candidates of the next window, of at
-// most kWindow gates from cnt->step on and before hi. Bound by memory: 16 bytes of coefficient per term and the columns of
-// the window's gates, against 64 bytes per anticommuting (term, gate) pair when done gate by gate. A warp
-// takes 8 column words: eight lanes form one gate's words (one 32-byte sector per column), the words go
-// through shared memory to a bit transposition, and every lane then holds the gate mask of its own term.
+// Applies the pending window (ctl) to its passive terms and collects the candidates of the next window, of at most
+// kWindow gates from cnt->step on and before hi. Bound by memory: 16 bytes of coefficient per term and the columns of
+// the window's gates, against 64 bytes per anticommuting (term, gate) pair when done gate by gate. A warp takes 8
+// column words: eight lanes form one gate's words (one 32-byte sector per column), the words go through shared memory
+// to a bit transposition, and every lane then holds the gate mask of its own term.
 __global__ void __launch_bounds__(kCloseWarps * 32, 4)
     k_window_close(Store st, uint32_t parity_col, WindowScratch ws, uint32_t *__restrict__ cand, const Counters *__restrict__ cnt,
                    const GateDesc *__restrict__ gates, uint32_t L, uint32_t hi, Trunc tr, uint64_t *__restrict__ stats) {
@@ -418,11 +419,11 @@ __global__ void __launch_bounds__(256) k_window_sample(Store st, WindowScratch w
 //   active term and 1.5 ps per term (measured from 1 to 3e6 terms: 5.6 us at a few terms, 12 at 3e5 with 2e4 active and
 //   anticommuting, 33 at 1e6 with 4e5).
 // Up to 1.15 times that, windows go on (a declined try and the way back cost as much), and 0.2 ms over the gates that
-// are left in favour of windows: what a change over costs.
-// Measured on lines and lattices, windows against gate by gate: 2.0 times as long over 8 gates, 1.2 over 32, 0.8 over 64; on 8
-// to 11 qubits without truncation, where no length but the shortest is balanced, 1.2 to 2.2. In whole numbers: every
-// block of the two kernels that ask (count, which makes the masks, and scatter, which sets the window up) has to come
-// to the same length, and floating-point sums may be contracted differently in each.
+// are left in favour of windows: what a change over costs. Measured on lines and lattices, windows against gate by
+// gate: 2.0 times as long over 8 gates, 1.2 over 32, 0.8 over 64; on 8 to 11 qubits without truncation, where no
+// length but the shortest is balanced, 1.2 to 2.2. In whole numbers: every block of the two kernels that ask (count,
+// which makes the masks, and scatter, which sets the window up) has to come to the same length, and floating-point
+// sums may be contracted differently in each.
 struct LengthShared {
     uint32_t most[kLengths], sum[kLengths];
 };
