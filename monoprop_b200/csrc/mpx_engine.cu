@@ -1781,6 +1781,19 @@ mpx_status build_plan(mpx_engine *eng, const CircuitDev &cd, const FrozenGraph &
     A(&so.busiest, n_win);
     A(&so.c_mask, places);
     A(&so.c_sector, places);
+    const bool ordered = &g == &e->fg; // a graph's gradients are the same bits on every call
+    std::vector<uint2> parts;
+    uint2 *d_parts = nullptr;
+    for (uint64_t st = 0; ordered && st < L; ++st) {
+        const uint32_t part0 = static_cast<uint32_t>(parts.size());
+        for (uint64_t k = 0; k < g.count[st]; k += kPlacePairs) parts.push_back(uint2{static_cast<uint32_t>(st), part0});
+    }
+    if (ordered) {
+        A(&d_parts, parts.size());
+        A(&so.tally, parts.size() * q.sectors);
+    }
+    if (ce == cudaSuccess && !parts.empty())
+        ce = cudaMemcpyAsync(d_parts, parts.data(), parts.size() * sizeof(uint2), cudaMemcpyHostToDevice, e->stream);
     if (ce == cudaSuccess)
         ce = cudaMemcpyAsync(so.base, base.data(), n_win * sizeof(uint32_t), cudaMemcpyHostToDevice, e->stream);
     const ReplayLaunch a = replay_launch(e, cd, g);
@@ -1795,14 +1808,15 @@ mpx_status build_plan(mpx_engine *eng, const CircuitDev &cd, const FrozenGraph &
     if (ce == cudaSuccess) ce = cudaStreamSynchronize(e->stream);
     for (const uint32_t b : busiest) work.busiest += b;
     const bool pays = replay_pays(work, most);
-    if (ce == cudaSuccess && pays && in_vs == nullptr) ce = replay_place(a, q, so, g.src, g.tgt, g.code, g.p_begin, g.p_count);
-    for (uint32_t w = 0; ce == cudaSuccess && pays && in_vs != nullptr && w < n_win; ++w)
+    if (ce == cudaSuccess && pays && ordered)
+        ce = replay_place(a, q, so, d_parts, static_cast<uint32_t>(parts.size()), g.src, g.tgt, g.code, g.p_begin, g.p_count);
+    for (uint32_t w = 0; ce == cudaSuccess && pays && !ordered && w < n_win; ++w)
         ce = replay_scatter(a, q, so, w, g.src, g.tgt, g.code, in_vs, in_vt, vs, vt, g.p_begin, g.p_count, begin[w * K],
                             range[w]);
-    e->launches += 2 + n_win + (!pays ? 0 : in_vs == nullptr ? 1 : n_win);
+    e->launches += 2 + n_win + (!pays ? 0 : ordered ? 2 : n_win);
     for (void *ptr : {static_cast<void *>(so.tables), static_cast<void *>(so.cursor), static_cast<void *>(so.base),
-                      static_cast<void *>(so.busiest), static_cast<void *>(so.c_mask),
-                      static_cast<void *>(so.c_sector)})
+                      static_cast<void *>(so.busiest), static_cast<void *>(so.c_mask), static_cast<void *>(so.c_sector),
+                      static_cast<void *>(so.tally), static_cast<void *>(d_parts)})
         dev_free(e, ptr);
     if (ce == cudaSuccess && !pays) {
         free_plan(e, q);

@@ -111,7 +111,7 @@ __global__ void __launch_bounds__(1024) k_replay_prefix(ReplayPlan p, ReplaySort
     if (threadIdx.x == 0) so.busiest[blockIdx.x] = s_most;
 }
 
-// Places the pairs and their logged values, in any order within a sector and gate: the log of a propagation has none
+// Places the pairs (and their logged values) in any order within a sector and gate: the log of a propagation has none
 // of its own.
 __global__ void __launch_bounds__(256) k_replay_scatter(ReplayPlan p, ReplaySort so, uint32_t window, uint32_t L,
                                                          const uint32_t *__restrict__ src, const uint32_t *__restrict__ tgt,
@@ -138,44 +138,91 @@ __global__ void __launch_bounds__(256) k_replay_scatter(ReplayPlan p, ReplaySort
         p.tgt[at] = tgt[r];
         p.code[at] = code[r];
         p.mask[at] = so.c_mask[r];
-        vs[at] = in_vs[r];
-        vt[at] = in_vt[r];
+        if (in_vs != nullptr) {
+            vs[at] = in_vs[r];
+            vt[at] = in_vt[r];
+        }
     }
 }
 
-// The same in the log's order, one block per gate: a structure that is replayed again and again keeps one order of its
-// pairs, whichever engine sorts it (a clone has the same log). Warps take their turns at the sectors' cursors, 32 pairs
-// a turn; a gate of 3e5 pairs takes about half a millisecond, once per structure.
-__global__ void __launch_bounds__(256) k_replay_place(ReplayPlan p, ReplaySort so, const uint32_t *__restrict__ src,
-                                                       const uint32_t *__restrict__ tgt, const int8_t *__restrict__ code,
+// The same in the log's order: a structure that is replayed again and again keeps one order of its pairs, whichever
+// engine sorts it (a clone has the same log). A gate's pairs are dealt to blocks in contiguous parts of kPlacePairs
+// (parts[b]: gate and first part of block b's gate), a part to warps in contiguous shares. Every warp has its own
+// cursor per sector: it counts, the counts become first places (after the parts before, whose counts
+// k_replay_tally left), and it places its share 32 pairs at a time, each pair after those of its sector that come
+// before it. Bound by the scattered stores of 17 bytes a pair; the next 32 are loaded ahead. The first gradient over
+// a new graph, sort included: 100 qubits (8 layers, 8e7 pairs) 35.1 ms, with one block per gate 43, in any order 33;
+// 50 qubits 10.7, 11.8 and 10.3 ms.
+constexpr int kPlaceWarps = 16;
+
+// Pairs per sector of every part that is not its gate's only or last one.
+__global__ void __launch_bounds__(256) k_replay_tally(uint32_t sectors, ReplaySort so, const uint2 *__restrict__ parts,
                                                        const uint64_t *__restrict__ p_begin,
                                                        const unsigned long long *__restrict__ p_count) {
-    __shared__ uint32_t s_cursor[kMaxSectors];
-    const uint32_t window = blockIdx.x / p.gates, g = blockIdx.x % p.gates;
-    const uint64_t first = p_begin[blockIdx.x], count = p_count[blockIdx.x];
-    if (count == 0) return;
-    const uint32_t *cursor = so.cursor + static_cast<uint64_t>(window) * p.sectors * p.gates;
-    for (uint32_t s = threadIdx.x; s < p.sectors; s += blockDim.x) s_cursor[s] = cursor[s * p.gates + g];
+    __shared__ uint32_t s_count[kMaxSectors];
+    const uint2 part = parts[blockIdx.x];
+    const uint64_t lo = static_cast<uint64_t>(blockIdx.x - part.y) * kPlacePairs, first = p_begin[part.x] + lo;
+    if (p_count[part.x] <= lo + kPlacePairs) return;
+    for (uint32_t s = threadIdx.x; s < sectors; s += blockDim.x) s_count[s] = 0;
+    __syncthreads();
+    for (uint32_t k = threadIdx.x; k < kPlacePairs; k += blockDim.x) atomicAdd(&s_count[so.c_sector[first + k]], 1u);
+    __syncthreads();
+    for (uint32_t s = threadIdx.x; s < sectors; s += blockDim.x) so.tally[static_cast<uint64_t>(blockIdx.x) * sectors + s] = s_count[s];
+}
+
+__global__ void __launch_bounds__(kPlaceWarps * 32)
+    k_replay_place(ReplayPlan p, ReplaySort so, const uint2 *__restrict__ parts, const uint32_t *__restrict__ src,
+                   const uint32_t *__restrict__ tgt, const int8_t *__restrict__ code, const uint64_t *__restrict__ p_begin,
+                   const unsigned long long *__restrict__ p_count) {
+    extern __shared__ uint32_t s_at[]; // [kPlaceWarps][sectors]
+    const uint2 part = parts[blockIdx.x];
+    const uint32_t window = part.x / p.gates, g = part.x % p.gates, S = p.sectors;
+    const uint64_t skip = static_cast<uint64_t>(blockIdx.x - part.y) * kPlacePairs, all = p_count[part.x];
+    if (all <= skip) return;
+    const uint64_t first = p_begin[part.x] + skip, count = min(all - skip, uint64_t(kPlacePairs));
+    for (uint32_t k = threadIdx.x; k < kPlaceWarps * S; k += blockDim.x) s_at[k] = 0;
     __syncthreads();
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (uint64_t k0 = 0; k0 < count; k0 += blockDim.x) {
-        const uint64_t r = first + k0 + threadIdx.x;
-        const bool in = k0 + threadIdx.x < count;
-        const uint32_t s = in ? so.c_sector[r] : kNoSector;
-        const uint32_t peers = __match_any_sync(0xFFFFFFFFu, s);
-        const uint32_t rank = __popc(peers & ((1u << lane) - 1u));
-        uint32_t at = 0;
-        for (uint32_t w = 0; w < blockDim.x / 32; ++w) {
-            if (w == warp && in) at = s_cursor[s] + rank;
-            __syncwarp();
-            if (w == warp && in && rank == 0) s_cursor[s] = at + __popc(peers);
-            __syncthreads();
+    const uint64_t share = ((count + kPlaceWarps - 1) / kPlaceWarps + 31) / 32 * 32;
+    const uint64_t lo = min(count, warp * share), hi = min(count, lo + share);
+    uint32_t *at = s_at + warp * S;
+    for (uint64_t k = lo + lane; k < hi; k += 32) atomicAdd(&at[so.c_sector[first + k]], 1u);
+    __syncthreads();
+    const uint32_t *cursor = so.cursor + static_cast<uint64_t>(window) * S * p.gates;
+    for (uint32_t s = threadIdx.x; s < S; s += blockDim.x) {
+        uint32_t acc = cursor[s * p.gates + g];
+        for (uint32_t b = part.y; b < blockIdx.x; ++b) acc += so.tally[static_cast<uint64_t>(b) * S + s];
+        for (int w = 0; w < kPlaceWarps; ++w) {
+            const uint32_t c = s_at[w * S + s];
+            s_at[w * S + s] = acc;
+            acc += c;
         }
-        if (in) {
-            p.src[at] = src[r];
-            p.tgt[at] = tgt[r];
-            p.code[at] = code[r];
-            p.mask[at] = so.c_mask[r];
+    }
+    __syncthreads();
+    struct Pair {
+        uint32_t sector, s, t;
+        int8_t code;
+        uint64_t mask;
+    };
+    auto load = [&](uint64_t k) {
+        const uint64_t r = first + k;
+        return k < hi ? Pair{so.c_sector[r], src[r], tgt[r], code[r], so.c_mask[r]} : Pair{kNoSector, 0, 0, 0, 0};
+    };
+    Pair next = load(lo + lane);
+    for (uint64_t k = lo + lane; k - lane < hi; k += 32) { // warp-uniform
+        const Pair q = next;
+        next = load(k + 32);
+        const uint32_t peers = __match_any_sync(0xFFFFFFFFu, q.sector), rank = __popc(peers & ((1u << lane) - 1u));
+        uint32_t place = 0;
+        if (k < hi) place = at[q.sector] + rank;
+        __syncwarp();
+        if (k < hi && rank == 0) at[q.sector] = place + __popc(peers);
+        __syncwarp();
+        if (k < hi) {
+            p.src[place] = q.s;
+            p.tgt[place] = q.t;
+            p.code[place] = q.code;
+            p.mask[place] = q.mask;
         }
     }
 }

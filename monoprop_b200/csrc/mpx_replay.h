@@ -34,7 +34,9 @@ struct ReplaySort {
     uint32_t *busiest;  // [windows] out: most pairs of one sector
     uint64_t *c_mask;
     uint16_t *c_sector;
+    uint32_t *tally;    // [parts][sectors] (replay_place)
 };
+constexpr uint32_t kPlacePairs = 1u << 15; // pairs per part
 
 cudaError_t replay_tables(const ReplayLaunch &a, const ReplayPlan &p, const ReplaySort &s);
 cudaError_t replay_count(const ReplayLaunch &a, const ReplayPlan &p, const ReplaySort &s, uint32_t window,
@@ -46,8 +48,10 @@ cudaError_t replay_scatter(const ReplayLaunch &a, const ReplayPlan &p, const Rep
                            const double *in_vt, double *vs, double *vt, const uint64_t *p_begin,
                            const unsigned long long *p_count, uint64_t first, uint64_t count);
 
-cudaError_t replay_place(const ReplayLaunch &a, const ReplayPlan &p, const ReplaySort &s, const uint32_t *src,
-                         const uint32_t *tgt, const int8_t *code, const uint64_t *p_begin, const unsigned long long *p_count);
+// The pairs in the log's order within a sector and gate. parts: [n_parts] the gate of every part and the gate's first part.
+cudaError_t replay_place(const ReplayLaunch &a, const ReplayPlan &p, const ReplaySort &s, const uint2 *parts, uint32_t n_parts,
+                         const uint32_t *src, const uint32_t *tgt, const int8_t *code, const uint64_t *p_begin,
+                         const unsigned long long *p_count);
 
 // One window forward: its pairs (vs, vt: logged when not null), then the dense pass over the n_end terms it
 // leaves; ck: the coefficients after the window, when not null. last: [terms] zero between windows.

@@ -126,9 +126,15 @@ cudaError_t replay_forward(const ReplayLaunch &a, const ReplayPlan &p, uint32_t 
     return cudaGetLastError();
 }
 
-cudaError_t replay_place(const ReplayLaunch &a, const ReplayPlan &p, const ReplaySort &s, const uint32_t *src,
-                         const uint32_t *tgt, const int8_t *code, const uint64_t *p_begin, const unsigned long long *p_count) {
-    k_replay_place<<<a.L, 256, 0, a.stream>>>(p, s, src, tgt, code, p_begin, p_count);
+cudaError_t replay_place(const ReplayLaunch &a, const ReplayPlan &p, const ReplaySort &s, const uint2 *parts, uint32_t n_parts,
+                         const uint32_t *src, const uint32_t *tgt, const int8_t *code, const uint64_t *p_begin,
+                         const unsigned long long *p_count) {
+    if (n_parts == 0) return cudaSuccess;
+    const size_t bytes = static_cast<size_t>(kPlaceWarps) * p.sectors * sizeof(uint32_t); // at most 128 KB (kMaxSectors)
+    const cudaError_t ce = cudaFuncSetAttribute(k_replay_place, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
+    if (ce != cudaSuccess) return ce;
+    k_replay_tally<<<n_parts, 256, 0, a.stream>>>(p.sectors, s, parts, p_begin, p_count);
+    k_replay_place<<<n_parts, kPlaceWarps * 32, bytes, a.stream>>>(p, s, parts, src, tgt, code, p_begin, p_count);
     return cudaGetLastError();
 }
 
