@@ -1335,6 +1335,7 @@ mpx_status run_range(mpx_engine *eng, const CircuitDev &cd, uint64_t lo, uint64_
             }
             else {
                 stretch = hi;
+                ran_as.back().to = hi; // windows were tried before
             }
         }
         if (step < stretch) {
