@@ -25,7 +25,13 @@ def only_free(nbytes):
     _native.load().mpx_trim_device_memory(0)
     torch.cuda.empty_cache()
     torch.cuda.synchronize()
-    hold = torch.empty(max(torch.cuda.mem_get_info()[0] - nbytes, 0), dtype=torch.uint8, device="cuda")
+    rest, hold = max(torch.cuda.mem_get_info()[0] - nbytes, 0), None
+    for _ in range(8):  # the last few MiB may not be had in one block
+        with contextlib.suppress(torch.cuda.OutOfMemoryError):
+            hold = torch.empty(rest, dtype=torch.uint8, device="cuda")
+            break
+        rest -= 16 * MIB
+    assert hold is not None
     try:
         yield
     finally:

@@ -58,10 +58,12 @@ def test_generators_on_few_modes_do_not_put_the_store_on_one_block(modes):
     eng, circ = graph(wl)
 
     def seconds(segment_gates):
-        eng.graph_gradient(circ, segment_gates=segment_gates)
-        t = time.perf_counter()
-        eng.graph_gradient(circ, segment_gates=segment_gates)
-        return time.perf_counter() - t
+        best = np.inf
+        for _ in range(5):
+            t = time.perf_counter()
+            eng.graph_gradient(circ, segment_gates=segment_gates)
+            best = min(best, time.perf_counter() - t)
+        return best
 
     windows, gate_by_gate = seconds(0), seconds(60)
     circ.close()
@@ -73,15 +75,18 @@ def test_propagation_on_few_modes_does_not_stay_on_one_block():
     """only_rotate_len_k = all slots changes nothing but the path: gate by gate. Windows in which one block takes the
     whole store, as it grows from one term to 1e6 in one coset, take some twenty times as long."""
     wl = on_few_modes(161, 10, 150, 3)
-    seconds, sizes = [], []
+    seconds, results = [], []
     for k in (None, 2 * wl.num_modes):
-        for _ in range(2):
+        best = np.inf
+        for _ in range(4):
             eng = _native.engine_for(wl)
             eng.set_only_rotate_len_k(k)
             t = time.perf_counter()
             eng.propagate(wl.gen_words(), wl.angles())
-            seconds.append(time.perf_counter() - t)
-            sizes.append((eng.size(), eng.expectation()))
+            best = min(best, time.perf_counter() - t)
+            result = (eng.size(), eng.expectation())
             eng.close()
-    assert sizes[1][0] == sizes[3][0] and abs(sizes[1][1] - sizes[3][1]) <= 1e-12
-    assert seconds[1] <= 5 * seconds[3]
+        seconds.append(best)
+        results.append(result)
+    assert results[0][0] == results[1][0] and abs(results[0][1] - results[1][1]) <= 1e-12
+    assert seconds[0] <= 5 * seconds[1]
